@@ -10,7 +10,9 @@
 //    lock-free union-find: a union hooks the larger root under the smaller
 //    one with a compare-and-swap, finds halve paths.  Every parent is at most
 //    its child, so each component's root is its smallest triangle id, in any
-//    schedule.
+//    schedule.  On the GPU a block first joins the edges inside its tile of
+//    consecutive triangles in shared memory (regions.cu), and body_hook's
+//    global unions are left to the edges between tiles.
 // 2. Breadth-first rounds over components across constrained edges: round
 //    L gives every unreached component next to a component of depth L the
 //    depth L + 1 (all writers of a round store the same value).
@@ -28,34 +30,42 @@ constexpr int ERR_NEIGHBOUR = 1;         // a neighbour id outside -1..n_tris-1
 constexpr int ERR_LIMIT = 2;             // a bounded loop ran out
 
 #ifdef __CUDA_ARCH__
-// Parent links change under other threads: read them from L2, not L1.
-__device__ __forceinline__ int load_link(const int* p) { return __ldcg(p); }
 __device__ __forceinline__ int cas_link(int* p, int cmp, int val) { return atomicCAS(p, cmp, val); }
 #else
-inline int load_link(const int* p) { return *p; }
 inline int cas_link(int* p, int cmp, int val) { int o = *p; if (o == cmp) *p = val; return o; }
 #endif
+
+// Parent links change under other threads, and a load may return an older
+// link (from L1): an older link still leads to an ancestor, so a find then
+// ends at a node that was a root, and uf_union's compare-and-swap decides.
+// Reading through L2 instead sent every find to the one line that holds the
+// root of almost all triangles (compress 203 us of it on the scale mesh).
 
 // Root of x's tree (path halving), or -1 if the bound ran out.
 __host__ __device__ __forceinline__ int uf_find(int* parent, int x) {
     for (int it = 0; it < kMaxSteps; ++it) {
-        int p = load_link(parent + x);
+        int p = parent[x];
         if (p == x) return x;
-        int gp = load_link(parent + p);
+        int gp = parent[p];
         if (gp != p) parent[x] = gp;     // gp is an ancestor of x: any interleaving keeps the tree
         x = gp;
     }
     return -1;
 }
 
+// Hook the larger root under the smaller node.  When the larger one is no
+// root any more, go on from the link that the compare-and-swap returned:
+// it is smaller, so the retries end.  (The smaller node need not be a root
+// still: every link goes to a smaller id, so no cycle can form.)
 __host__ __device__ __forceinline__ int uf_union(int* parent, int a, int b) {
     for (int it = 0; it < kMaxSteps; ++it) {
         int ra = uf_find(parent, a), rb = uf_find(parent, b);
         if (ra < 0 || rb < 0) return ERR_LIMIT;
         if (ra == rb) return 0;
         if (ra < rb) { int t = ra; ra = rb; rb = t; }
-        if (cas_link(parent + ra, ra, rb) == ra) return 0;
-        a = ra;
+        const int was = cas_link(parent + ra, ra, rb);
+        if (was == ra) return 0;
+        a = was;
         b = rb;
     }
     return ERR_LIMIT;
@@ -67,13 +77,16 @@ __host__ __device__ __forceinline__ void body_init(int t, int* parent, int* leve
 }
 
 // Join triangle t with each neighbour of larger id across an unconstrained
-// edge (so every edge is joined once); check the neighbour ids.
-__host__ __device__ __forceinline__ int body_hook(const int* adj, const uint8_t* cf, int nt, int t, int* parent) {
+// edge (so every edge is joined once); check the neighbour ids.  `tile` > 0:
+// the neighbours in t's own tile of that many triangles are joined already.
+__host__ __device__ __forceinline__ int body_hook(const int* adj, const uint8_t* cf, int nt, int t, int* parent,
+                                                  int tile = 0) {
     int err = 0;
     for (int k = 0; k < 3; k++) {
         int u = adj[3ll * t + k];
         if (u == -1) continue;
         if ((unsigned)u >= (unsigned)nt) { err |= ERR_NEIGHBOUR; continue; }
+        if (tile > 0 && u / tile == t / tile) continue;
         if (u > t && !((cf[t] >> k) & 1)) err |= uf_union(parent, t, u);
     }
     return err;
@@ -82,7 +95,7 @@ __host__ __device__ __forceinline__ int body_hook(const int* adj, const uint8_t*
 // Root of x's tree without changing any link, or -1 if the bound ran out.
 __host__ __device__ __forceinline__ int uf_root(const int* parent, int x) {
     for (int it = 0; it < kMaxSteps; ++it) {
-        int p = load_link(parent + x);
+        int p = parent[x];
         if (p == x) return x;
         x = p;
     }
@@ -112,7 +125,7 @@ __host__ __device__ __forceinline__ void body_seed(const int* adj, int t, const 
 // constrained edges.  Returns 1 if it set any depth.
 __host__ __device__ __forceinline__ int body_expand(const int* adj, const uint8_t* cf, int nt, int t, int L,
                                                     const int* parent, int* level) {
-    if (level[parent[t]] != L) return 0;
+    if (!(cf[t] & 7) || level[parent[t]] != L) return 0;
     int changed = 0;
     for (int k = 0; k < 3; k++) {
         int u = adj[3ll * t + k];

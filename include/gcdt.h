@@ -254,7 +254,7 @@ gcdt_status gcdt_reference_layout(const int32_t* d_points, int32_t n,
    greatest depth.  d_scratch (256-byte aligned) holds at least
    gcdt_classify_regions_scratch_bytes(n_tris) bytes and must not overlap
    d_depth.  Runs on the current device; returns when d_depth is complete on
-   `stream` (one 4-byte read back per depth level).  GCDT_BAD_INPUT for a
+   `stream` (one 16-byte read back per two depth levels).  GCDT_BAD_INPUT for a
    neighbour id outside -1..n_tris-1, GCDT_OOM for too little scratch. */
 size_t gcdt_classify_regions_scratch_bytes(int32_t n_tris);
 gcdt_status gcdt_classify_regions(const int32_t* d_adj, const uint8_t* d_cflags, int32_t n_tris,

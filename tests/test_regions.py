@@ -177,6 +177,34 @@ def test_gpu_classification_equals_checker(case):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rings,npts", [(1, 1022), (2, 1023), (3, 1024), (4, 2047), (5, 3100)])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_gpu_classification_across_tiles(rings, npts, shuffled):
+    """Meshes whose triangle counts lie around whole tiles of 2,048, with
+    depths on both sides of the two rounds per read-back; shuffled triangle
+    numbers make almost every edge leave its tile."""
+    import torch
+    m = 24 * rings
+    ang = 2 * np.pi * np.arange(24) / 24
+    ring = [np.stack([np.cos(ang), np.sin(ang)], 1) * (1 << 28) * (k + 1) / (rings + 1) + (1 << 29) for k in range(rings)]
+    rng = np.random.default_rng(rings)
+    extra = rng.integers(1, (1 << 30) - 2, size=(npts - m, 2))
+    xy = np.concatenate([np.rint(np.concatenate(ring)), extra]).astype(np.int32)
+    assert len(np.unique(xy, axis=0)) == npts
+    cons = np.array([(24 * k + i, 24 * k + (i + 1) % 24) for k in range(rings) for i in range(24)], np.int32)
+    tris, adj, cf = _mesh(xy, cons)
+    if shuffled:
+        new = rng.permutation(len(adj))
+        old = np.argsort(new)
+        adj = np.where(adj[old] >= 0, new[adj[old]], -1).astype(np.int32)
+        cf = np.ascontiguousarray(cf[old])
+    want, wmd = regions.region_depth(adj, cf)
+    assert wmd == rings
+    depth, md = g.classify_regions(torch.from_numpy(np.ascontiguousarray(adj)).cuda(), torch.from_numpy(cf).cuda())
+    assert md == wmd and np.array_equal(depth.cpu().numpy(), want)
+
+
+@pytest.mark.gpu
 def test_gpu_classification_at_scale_equals_host_bodies():
     """The 10.2M-point scale mesh (20.4M triangles, 3,125 disjoint star
     polygons): the device's concurrent union-find must label every triangle
