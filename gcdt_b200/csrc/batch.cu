@@ -64,11 +64,9 @@ __global__ void gcdt_batch_keys(const int2* xy, const int* offs, int ninst, int 
     vals[g] = g - offs[lo];
 }
 
-template <int BS>
-__global__ void __launch_bounds__(BS) gcdt_batch_solve(BatchArgs a) {
-    const int inst = a.order[blockIdx.x];
-    BatchDesc d = a.desc[inst];
-    if (d.status) return;                        // rejected by the key pass
+// Instance `inst`'s context, over its slice of the arena.
+__device__ inline Ctx instance_ctx(const BatchArgs& a, int inst) {
+    const BatchDesc d = a.desc[inst];
     Plan p = make_plan(d.n, d.s, 0);
     Ctx c = bind_ctx(a.ws + d.ws_off, p);
     c.keys = const_cast<unsigned long long*>(a.keys) + d.pt_off;
@@ -78,22 +76,18 @@ __global__ void __launch_bounds__(BS) gcdt_batch_solve(BatchArgs a) {
     c.out_tris = a.tris + 3 * d.tri_off;
     c.out_adj = a.adj + 3 * d.tri_off;
     c.out_cflags = a.cflags + d.tri_off;
-    // small instances: two levels, the autotuned sample stride, then the rest
+    // small instances: two levels, the autotuned sample stride, then the
+    // rest, and no flip carried across rounds
     c.nlevels = 2;
     c.stride[0] = a.stride0; c.stride[1] = 1;
-    // the phases' items read the instance's context from shared memory, the
-    // fields the driver changes from its own copy (42.7k vs 40.5k instances/s
-    // on 4,096 instances, against a per-thread copy in local memory)
-    __shared__ Ctx sc;
-    if (threadIdx.x == 0) sc = c;
-    __syncthreads();
-    BlockExecT<true> ex{c.cnt, &sc};
-    // per-solve reset: counters and the per-triangle state
-    {
-        int* w = reinterpret_cast<int*>(c.cnt);
-        for (int k = threadIdx.x; k < (int)(sizeof(Counters) / 4); k += blockDim.x) w[k] = 0;
-        __syncthreads();
-    }
+    c.carry_q = 0;
+    return c;
+}
+
+// The whole solve of one instance, by its block's or cluster's driver warps;
+// returns the status bits.
+template <class EX>
+__device__ int solve_instance(EX& ex, const Ctx& c) {
     ex.phase(K_CLEAR, c, c.ntri);
     ex.phase(K_GATHER, c, c.n + 4);
     ex.phase(K_ROOT, c, 1);
@@ -103,19 +97,105 @@ __global__ void __launch_bounds__(BS) gcdt_batch_solve(BatchArgs a) {
         ex.phase(K_SEG_LEVEL0, c, c.s);
     }
     int st = ex.word(&c.cnt->err[0]) | ex.word(&c.cnt->err[1]) | ex.word(&c.cnt->status);
-    if (st == 0) {
-        run_stages(ex, c);
-        st = ex.word(&c.cnt->err[0]) | ex.word(&c.cnt->err[1]) | ex.word(&c.cnt->status);
-    }
+    return st ? st : run_stages(ex, c);
+}
+
+// BS threads, the last warp the driver.  What bounds an instance is latency
+// (its mesh sits in L2), so two blocks of 512 threads share an SM at 64
+// registers: 4,096 instances 86.8 -> 67.1 ms against one block at 128, and
+// three at 40 registers spill (67.6).
+template <int BS>
+__global__ void __launch_bounds__(BS, 1024 / BS) gcdt_batch_solve(BatchArgs a, int first) {
+    const int inst = a.order[first + blockIdx.x];
+    if (a.desc[inst].status) return;             // rejected by the key pass
+    __shared__ BlockShared<BS - 32> sh;
     if (threadIdx.x == 0) {
-        // run_stages' result is folded into cnt->status by BlockExec::finish
-        a.desc[inst].status = st | ex.word(&c.cnt->status);
+        sh.ctx = instance_ctx(a, inst);
+        sh.ctx.cnt = reinterpret_cast<Counters*>(sh.head);
     }
+    __syncthreads();
+    if (threadIdx.x < BS - 32) {
+        for (;;) {
+            block_sync(kBarWork);
+            if (sh.kind == kExit) return;
+            block_items(sh);
+            block_sync(kBarDone);
+        }
+    }
+    Ctx c = sh.ctx;
+    BlockExecT<BlockShared<BS - 32>> ex(sh, c);
+    Driver D;
+    memset(&D, 0, sizeof D);
+    ex.begin(D);
+    const int st = solve_instance(ex, c);
+    if (threadIdx.x == BS - 32) a.desc[inst].status = st;
+    publish(sh, kExit, c, 0, true);
+    block_sync(kBarWork);
+}
+
+// A cluster phase's items read the context from shared memory; its lists are
+// in device memory.
+struct SharedView {
+    const Ctx& ctx;
+    template <int K> __device__ __forceinline__ Ctx items() const {
+        Ctx c = items_view(ctx, K);
+        __builtin_assume(__isGlobal(c.cnt));
+        if constexpr (K == K_FLIP_CHECK || K == K_FLIP_DO || K == K_FLIP_FIX) {
+            __builtin_assume(__isGlobal(c.cand));
+            if constexpr (K != K_FLIP_DO) __builtin_assume(__isGlobal(c.queue));
+            if constexpr (K != K_FLIP_CHECK) __builtin_assume(__isGlobal(c.queue_next));
+        } else if constexpr (K == K_FIX) {
+            __builtin_assume(__isGlobal(c.winners));
+            __builtin_assume(__isGlobal(c.queue_next));
+        } else {
+            __builtin_assume(__isGlobal(c.act));
+            if constexpr (K == K_SPLIT) __builtin_assume(__isGlobal(c.winners));
+            else __builtin_assume(__isGlobal(c.act_next));
+        }
+        return c;
+    }
+    __device__ __forceinline__ const Ctx& other() const { return ctx; }
+};
+
+// One instance per cluster, for instances that would be longer than the rest
+// of the batch in one block.  The blocks are as large as the single ones, so
+// that either fills the room the other leaves.
+constexpr int kClusterThreads = 512;
+__global__ void __launch_bounds__(kClusterThreads, 2) gcdt_batch_cluster(BatchArgs a, int first) {
+    const unsigned rank = cluster_rank(), size = cluster_size();
+    const int inst = a.order[first + blockIdx.x / size];
+    if (a.desc[inst].status) return;             // rejected by the key pass
+    constexpr int kWork = kClusterThreads - 32;
+    using SH = BlockShared<kWork>;
+    __shared__ SH sh;
+    if (threadIdx.x == 0) sh.ctx = instance_ctx(a, inst);
+    __syncthreads();
+    Counters* cnt = sh.ctx.cnt;
+    if (rank == 0 && threadIdx.x < kWork)
+        for (int k = threadIdx.x; k < (int)(sizeof(Counters) / 8); k += kWork)
+            reinterpret_cast<unsigned long long*>(cnt)[k] = 0;
+    __syncthreads();
+    cluster_sync();
+    if (threadIdx.x < kWork) {
+        team_worker<true, 1>(sh, rank, size, SharedView{sh.ctx});
+        return;
+    }
+    Ctx c = sh.ctx;
+    TeamExec<true, SH> ex{cnt, rank, size, &sh};
+    ex.take_snapshot();
+    const int st = solve_instance(ex, c);
+    if (rank == 0 && threadIdx.x == kWork) a.desc[inst].status = st;
+    publish(sh, kExit, c, 0, false);
+    block_sync(kBarWork);
 }
 
 }  // namespace gcdt
 
 using namespace gcdt;
+
+namespace {
+constexpr int kClusterSizes = 3;     // of 8, 4 and 2 blocks
+}
 
 struct gcdt_batch {
     int device = 0;
@@ -133,6 +213,10 @@ struct gcdt_batch {
     int* h_order = nullptr;          // pinned
     gcdt_batch_config cfg{256, 64};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // the clusters' launches run beside the single blocks': one stream and
+    // event per cluster size
+    cudaStream_t side[kClusterSizes] = {};
+    cudaEvent_t fork = nullptr, join[kClusterSizes] = {};
     double last_ms = 0.0;
 };
 
@@ -159,6 +243,19 @@ size_t arena_bound(int64_t max_inst, int64_t max_pts, int64_t max_segs) {
     // alignment per array: bound the sum over instances by the totals plus
     // one empty instance's layout and 48 alignment pads per instance.
     return make_plan(max_pts, max_segs, 0).L.total + (size_t)max_inst * (instance_bytes(0, 0) + 48 * 256);
+}
+
+// Blocks for an instance of n points in a batch of `total`: enough that it
+// takes no longer than the whole batch does on the GPU's 296 half-SM blocks.
+// 256 instances of 64 to 65,536 points (2.4M in all; one block for the
+// largest takes 13.5 ms): 14.5 -> 7.7 ms with the share at total / 200, 8.4
+// at / 160 and 8.0 at / 240.  Below 2,000 points a block's fast commands
+// (exec.cuh) do most of the work and a cluster has nothing to share.
+constexpr int64_t kClusterMinPoints = 2000, kShares = 200;
+int cluster_blocks(int64_t n, int64_t total) {
+    if (n < kClusterMinPoints) return 1;
+    const int64_t share = total / kShares;
+    return n > 4 * share ? 8 : n > 2 * share ? 4 : n > share ? 2 : 1;
 }
 
 bool valid_cfg(const gcdt_batch_config& c) {
@@ -253,12 +350,50 @@ gcdt_status gcdt_batch_launch(gcdt_batch* b, int32_t ninst, const int64_t* pt_of
     a.adj = d_adj;
     a.cflags = d_cflags;
     a.stride0 = cfg.sample_stride;
-    switch (cfg.threads_per_instance) {
-    case 128: gcdt_batch_solve<128><<<ninst, 128, 0, st>>>(a); break;
-    case 512: gcdt_batch_solve<512><<<ninst, 512, 0, st>>>(a); break;
-    default: gcdt_batch_solve<256><<<ninst, 256, 0, st>>>(a); break;
+    // The largest instances, one per cluster, on streams of their own next
+    // to the other instances' blocks; the instances are in order of size.
+    cudaError_t e = cudaSuccess;
+    int at = 0;
+    bool forked = false, joined[kClusterSizes] = {};
+    for (int k = 0; k < kClusterSizes && e == cudaSuccess; ++k) {
+        const int size = 8 >> k;
+        int end = at;
+        while (end < ninst && cluster_blocks(b->h_desc[b->h_order[end]].n, total) >= size) ++end;
+        if (end == at) continue;
+        if (!forked) e = cudaEventRecord(b->fork, st);
+        forked = true;
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(b->side[k], b->fork, 0);
+        if (e != cudaSuccess) break;
+        joined[k] = true;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = size;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3((unsigned)(end - at) * size);
+        lc.blockDim = dim3(kClusterThreads);
+        lc.stream = b->side[k];
+        lc.attrs = attr;
+        lc.numAttrs = 1;
+        e = cudaLaunchKernelEx(&lc, gcdt_batch_cluster, a, at);
+        at = end;
     }
-    if (cudaGetLastError() != cudaSuccess) return GCDT_CUDA_ERROR;
+    if (e == cudaSuccess && at < ninst) {
+        const int m = ninst - at;
+        switch (cfg.threads_per_instance) {
+        case 128: gcdt_batch_solve<128><<<m, 128, 0, st>>>(a, at); break;
+        case 512: gcdt_batch_solve<512><<<m, 512, 0, st>>>(a, at); break;
+        default: gcdt_batch_solve<256><<<m, 256, 0, st>>>(a, at); break;
+        }
+        e = cudaGetLastError();
+    }
+    for (int k = 0; k < kClusterSizes; ++k) {
+        if (!joined[k]) continue;
+        cudaError_t j = cudaEventRecord(b->join[k], b->side[k]);
+        if (j == cudaSuccess) j = cudaStreamWaitEvent(st, b->join[k], 0);
+        if (e == cudaSuccess) e = j;
+    }
+    if (e != cudaSuccess) return GCDT_CUDA_ERROR;
     cudaMemcpyAsync(b->h_desc, b->d_desc, sizeof(BatchDesc) * ninst, cudaMemcpyDeviceToHost, st);
     return GCDT_OK;
 }
@@ -313,7 +448,11 @@ extern "C" gcdt_status gcdt_batch_create(gcdt_batch** out, int device, int64_t m
               cudaMallocHost(&b->h_desc, sizeof(BatchDesc) * max_instances) == cudaSuccess &&
               cudaMallocHost(&b->h_offs, 4 * (max_instances + 1)) == cudaSuccess &&
               cudaMallocHost(&b->h_order, 4 * max_instances) == cudaSuccess &&
-              cudaEventCreate(&b->ev0) == cudaSuccess && cudaEventCreate(&b->ev1) == cudaSuccess;
+              cudaEventCreate(&b->ev0) == cudaSuccess && cudaEventCreate(&b->ev1) == cudaSuccess &&
+              cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) == cudaSuccess;
+    for (int k = 0; k < kClusterSizes; ++k)
+        ok = ok && cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         gcdt_batch_destroy(b);
@@ -337,6 +476,11 @@ extern "C" void gcdt_batch_destroy(gcdt_batch* b) {
     if (b->h_order) cudaFreeHost(b->h_order);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
+    if (b->fork) cudaEventDestroy(b->fork);
+    for (int k = 0; k < kClusterSizes; ++k) {
+        if (b->side[k]) cudaStreamDestroy(b->side[k]);
+        if (b->join[k]) cudaEventDestroy(b->join[k]);
+    }
     delete b;
 }
 

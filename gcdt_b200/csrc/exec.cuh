@@ -1,10 +1,22 @@
-// exec.cuh -- the two executors of the stage driver on the GPU.
+// exec.cuh -- the executors of the stage driver on the GPU.
 //
-//   GridExec   every block of a cooperative persistent launch: a phase is a
-//              grid-stride loop followed by a bounded grid barrier;
-//   BlockExec  one block: a phase is a block-stride loop followed by
-//              __syncthreads (the single-block tails of a solve, and every
-//              instance of the batched path).
+// Every block is one driver warp and a number of worker warps.  The driver
+// warp runs the stage driver (solver.cuh); the workers run the phases' items:
+// the driver publishes a phase in shared memory, a block barrier releases the
+// workers, another one tells the driver that they are done.  So the driver's
+// state costs the items no registers (its path through the kernel is a
+// separate one), and its control words (list cursors, error words) can live
+// next to it.
+//
+//   TeamExec   the driver of every block of a team of blocks: a phase is a
+//              team-stride loop followed by a team barrier.  A team is the
+//              grid of a cooperative persistent launch (GridExec, bounded
+//              barrier on a counter) or a thread-block cluster (ClusterExec,
+//              the hardware's cluster barrier);
+//   BlockExec  the driver of one block: a phase is a block-stride loop (the
+//              single-block tails of a solve, and every instance of the
+//              batched path), with the counters and the short lists in
+//              shared memory.
 #pragma once
 #include "solver.cuh"
 
@@ -16,18 +28,21 @@ namespace gcdt {
 // grid-stride loops separated by a grid barrier, so the round structure
 // costs no kernel launches and no host round trips.
 
-#ifndef GCDT_PERSIST_BLOCK
-#define GCDT_PERSIST_BLOCK 512
+#ifndef GCDT_STAGE_WORKERS
+#define GCDT_STAGE_WORKERS 19
 #endif
-#ifndef GCDT_PERSIST_MINB
-#define GCDT_PERSIST_MINB 1
-#endif
-constexpr int kPersistBlock = GCDT_PERSIST_BLOCK;   // 512: one block per SM (128 registers per thread)
-constexpr int kPersistMinBlocks = GCDT_PERSIST_MINB;
+// Worker warps per block, one block per SM.  The phases are bound by the
+// latency of dependent loads, so by loads in flight per SM: 20 warps at 96
+// registers with two queue entries per thread (21.5 ms on the headline
+// solve) against 16 warps at 128 (22.7 with the driver in every thread),
+// 24 at 80 (22.4), 28 at 72 and one entry (22.9), 32 at 64 (25.1; 23.7 with
+// one entry): below 96 registers the flip passes spill.
+constexpr int kStageWorkers = GCDT_STAGE_WORKERS;
+constexpr int kPersistBlock = 32 * (kStageWorkers + 1);    // and the driver warp, the last one
 
 // The context a phase's items see: the launch's context `param` (in kernel
 // parameter space) with the fields the driver changes between phases taken
-// from the driver's copy `c`.  The other fields (the array pointers and
+// from the published copy `c`.  The other fields (the array pointers and
 // sizes) stay reads of parameter space, so the item loops keep them in no
 // register.
 __device__ __forceinline__ Ctx phase_view(const Ctx& param, const Ctx& c) {
@@ -38,30 +53,565 @@ __device__ __forceinline__ Ctx phase_view(const Ctx& param, const Ctx& c) {
     v.pend = c.pend; v.pend_next = c.pend_next; v.lq = c.lq;
     v.base_act = c.base_act; v.base_win = c.base_win; v.base_q = c.base_q; v.base_flip = c.base_flip;
     v.base_pend = c.base_pend; v.base_law = c.base_law; v.base_scr = c.base_scr;
+    // the grid's lists are all in device memory (a block's may be in shared)
+    __builtin_assume(__isGlobal(v.act)); __builtin_assume(__isGlobal(v.act_next));
+    __builtin_assume(__isGlobal(v.queue)); __builtin_assume(__isGlobal(v.queue_next));
+    __builtin_assume(__isGlobal(v.pend)); __builtin_assume(__isGlobal(v.pend_next));
+    __builtin_assume(__isGlobal(v.lq));
     return v;
 }
 
-struct GridExec {
+// ---------------------------------------------------------------- a block
+
+// The head of Counters: status, error words and list cursors.
+constexpr int kSnapWords = 12;
+static_assert(offsetof(Counters, cur_scr) + 8 <= kSnapWords * 8, "cursors are in the snapshot");
+
+constexpr int kExit = -1;            // published kinds besides the phases: the kernel ends,
+constexpr int kFastFlips = 100;      // whole flip sub-rounds on a short queue,
+constexpr int kFastRound = 101;      // an insertion round of a short active list,
+constexpr int kTeamSync = 102;       // nothing but the team barrier (clusters)
+
+// What the driver warp and the workers of a block share.  CAP: entries of
+// the lists a single-block phase keeps here, and the threads (one item each)
+// of the fast commands.
+template <int CAP>
+struct BlockShared {
+    static constexpr int kCap = CAP;
+    Ctx ctx;                    // the launch's context with the running phase's fields
+    long long count;            // items of the phase
+    int kind;                   // phase kind
+    int single;                 // the items run on this block alone
+    int work;                   // next chunk of the phase (dynamic phases)
+    unsigned long long head[kSnapWords];   // BlockExec's counters
+    alignas(16) int queue[2][4 * CAP];      // short flip queues (an insertion of CAP points makes at most 4 CAP)
+    alignas(16) int2 cand[CAP];
+    int act[2][CAP];
+    int2 winners[CAP];
+    // the fast commands' lists (see fast_flips, fast_round)
+    int budget;                 // flip sub-rounds they may take
+    int tally[3][2];            // flips and losers of a sub-round, in turn of three
+    int n_alive, n_won, n_next; // active points, inserted points and survivors of a round
+    int n_queue;                // entries of the flip queue they leave
+    int subrounds, flips;       // sub-rounds and flips they took
+};
+
+// Block barriers 1 (phase published) and 2 (items done); every thread of the
+// block takes part in both.
+__device__ __forceinline__ void block_sync(int id) {
+    asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(blockDim.x) : "memory");
+}
+constexpr int kBarWork = 1, kBarDone = 2;
+
+// Publish the fields of c that phase k's items read (driver warp; lane 0
+// writes).  The lists and the counters are among them each time: a
+// single-block phase's are in shared memory, a team phase's never are.
+template <class SH>
+__device__ __forceinline__ void publish(SH& sh, int k, const Ctx& c, long long count, bool single) {
+    if ((threadIdx.x & 31) == 0) {
+        Ctx& v = sh.ctx;
+        sh.kind = k; sh.count = count; sh.single = single; sh.work = 0;
+        v.round = c.round; v.sr = c.sr; v.eslot = c.eslot; v.cnt = c.cnt;
+        if (k == K_FLIP_CHECK || k == K_FLIP_DO || k == K_FLIP_FIX) {
+            v.list_n = c.list_n; v.carry_n = c.carry_n;
+            v.queue = c.queue; v.queue_next = c.queue_next; v.cand = c.cand;
+            v.base_q = c.base_q; v.base_flip = c.base_flip;
+        } else if (k == kFastFlips) {
+            v.queue = c.queue; v.carry_n = c.carry_n;
+        } else if (k == K_RELOC_VOTE || k == K_SPLIT || k == K_FIX || k == kFastRound) {
+            v.act = c.act; v.act_next = c.act_next; v.queue_next = c.queue_next; v.winners = c.winners;
+            v.base_act = c.base_act; v.base_win = c.base_win; v.base_q = c.base_q;
+        } else {
+            v.level = c.level; v.lawson_sr = c.lawson_sr;
+            v.act_next = c.act_next; v.base_act = c.base_act;
+            v.pend = c.pend; v.pend_next = c.pend_next; v.lq = c.lq;
+            v.base_pend = c.base_pend; v.base_law = c.base_law; v.base_scr = c.base_scr;
+        }
+    }
+    __syncwarp();
+}
+
+// Driver of one block (see above).  Its lists: a phase of at most CAP items
+// writes its list to shared memory, a longer one to the list's array; cur_*
+// say where the current one is.
+template <class SH>
+struct BlockExecT {
+    static constexpr bool kCanNarrow = false;
+    static constexpr int kFastItems = SH::kCap;
+    SH& sh;
+    int2* const all_cand;       // the lists' arrays
+    int2* const all_winners;
+    int* cur_act = nullptr;
+    int* cur_q = nullptr;
+    int2* cur_win = nullptr;
+    int2* cur_cand = nullptr;
+    int* nxt_q = nullptr;
+
+    __device__ BlockExecT(SH& s, const Ctx& c) : sh(s), all_cand(c.cand), all_winners(c.winners) {}
+    // The block's counters, at the driver's cursors.
+    __device__ Counters* begin(const Driver& D) {
+        Counters* cnt = reinterpret_cast<Counters*>(sh.head);
+        if ((threadIdx.x & 31) == 0) {
+            for (int k = 0; k < kSnapWords; ++k) sh.head[k] = 0;
+            cnt->cur_act0 = D.e_act0; cnt->cur_act = D.e_act; cnt->cur_win = D.e_win; cnt->cur_q = D.e_q;
+            cnt->cur_flip = D.e_flip; cnt->cur_pend = D.e_pend; cnt->cur_law = D.e_law; cnt->cur_scr = D.e_scr;
+        }
+        __syncwarp();
+        return cnt;
+    }
+    __device__ void phase(int k, const Ctx& cd, long long count) {
+        Ctx c = cd;
+        const bool fits = count <= SH::kCap;
+        c.cand = all_cand; c.winners = all_winners;
+        switch (k) {
+        case K_ACTIVATE: cur_act = c.act_next; break;
+        case K_RELOC_VOTE:
+            c.act = cur_act;
+            if (fits) c.act_next = sh.act[cur_act == sh.act[0]];
+            cur_act = c.act_next;
+            break;
+        case K_SPLIT:
+            c.act = cur_act;
+            if (fits) c.winners = sh.winners;
+            cur_win = c.winners;
+            break;
+        case K_FIX:
+            c.winners = cur_win;
+            if (fits) c.queue_next = sh.queue[0];
+            cur_q = c.queue_next;
+            break;
+        case K_FLIP_CHECK:
+            c.queue = cur_q;
+            cur_cand = fits ? sh.cand : c.cand;
+            c.cand = cur_cand;
+            break;
+        case K_FLIP_DO:
+            if (fits) c.queue_next = sh.queue[cur_q == sh.queue[0]];
+            nxt_q = c.queue_next;
+            c.cand = cur_cand;
+            break;
+        case K_FLIP_FIX:
+            c.queue = cur_q; c.queue_next = nxt_q; c.cand = cur_cand;
+            cur_q = nxt_q;
+            break;
+        case K_CPROC: cur_q = c.lq; break;
+        default: break;
+        }
+        run(k, c, count);
+    }
+    __device__ void run(int k, const Ctx& c, long long count) {
+        publish(sh, k, c, count, true);
+        block_sync(kBarWork);
+        block_sync(kBarDone);
+    }
+    // Flip sub-rounds on a queue of nq <= CAP entries, until it is empty, or
+    // longer than CAP, or `left` sub-rounds are used up (left counts down).
+    __device__ int fast_flips(Ctx& c, Driver& D, long long& nq, long long& left) {
+        c.sr = D.sr;
+        c.queue = cur_q;
+        c.carry_n = (int)D.drop;
+        D.drop = 0;
+        if ((threadIdx.x & 31) == 0) sh.budget = (int)left;
+        run(kFastFlips, c, nq);
+        const int took = sh.subrounds, nf = sh.flips;
+        cur_q = sh.queue[(cur_q == sh.queue[0]) ^ ((took + 1) & 1)];
+        left -= took;
+        D.sr += took;
+        D.subrounds += took;
+        D.e_flip += nf;
+        if ((threadIdx.x & 31) == 0) c.cnt->cur_flip = D.e_flip;
+        nq = sh.n_queue;
+        D.errs |= word(&c.cnt->err[c.eslot]);
+        return D.errs;
+    }
+    // One insertion round of nact <= CAP active points: returns the number
+    // of points that were still active, and leaves the survivors in nact and
+    // the flip queue's length in nq.
+    __device__ int fast_round(Ctx& c, Driver& D, long long& nact, long long& nq) {
+        c.act = cur_act;
+        c.act_next = sh.act[cur_act == sh.act[0]];
+        c.queue_next = sh.queue[0];
+        run(kFastRound, c, nact);
+        cur_act = c.act_next;
+        cur_q = sh.queue[0];
+        nact = sh.n_next;
+        nq = sh.n_queue;
+        D.errs |= word(&c.cnt->err[c.eslot]);
+        return sh.n_alive;
+    }
+    // Leave the first n entries of the current flip queue in q.
+    __device__ void store_queue(int* q, long long n) {
+        if (cur_q == q) return;
+        for (long long i = threadIdx.x & 31; i < n; i += 32) q[i] = cur_q[i];
+        __syncwarp();
+    }
+    __device__ unsigned long long cursor(unsigned long long* p) { return *(volatile unsigned long long*)p; }
+    __device__ int word(int* p) { return *(volatile int*)p; }
+    __device__ void finish(const Ctx& c, long long, long long, long long, int rc) {
+        if ((threadIdx.x & 31) == 0 && rc) c.cnt->status |= rc;
+        __syncwarp();
+    }
+    __device__ int narrow_flips(Ctx&, Driver&, long long&) { return ST_INTERNAL; }
+    __device__ int narrow_rounds(Ctx&, Driver&, long long) { return ST_INTERNAL; }
+};
+
+// Short lists.  With at most one item per thread, whole sub-rounds and rounds
+// run without the driver, an item's state staying in its thread's registers
+// from one phase to the next: the flipping thread resolves its own flip's
+// outer edges, a point's thread splits and resolves it.  These lists decide
+// the time of a solve of up to about 100,000 points and the tails of every
+// level; their phases are a few hundred dependent instructions on a few
+// warps, so publishing each phase, its lists in memory and generic
+// addressing cost more than its work (a flip sub-round of the tails 5.6 -> 2.2 us: check 1.1, flip 0.45, fix
+// 0.65; a round's insertion 9 -> 4.8 us).
+
+constexpr int kBarFast = 3;
+template <int CAP>
+__device__ __forceinline__ void fast_sync() {
+    asm volatile("bar.sync %0, %1;" :: "n"(kBarFast), "n"(CAP) : "memory");
+}
+
+// The fields of the published context that the fast commands use.
+__device__ __forceinline__ Ctx fast_view(const Ctx& p) {
+    Ctx c{};
+    c.n = p.n; c.ntri = p.ntri; c.round = p.round; c.sr = p.sr; c.eslot = p.eslot;
+    c.P = p.P; c.tri = p.tri; c.claim = p.claim; c.vote = p.vote; c.loc = p.loc; c.cnt = p.cnt;
+    __builtin_assume(__isGlobal(c.P)); __builtin_assume(__isGlobal(c.tri)); __builtin_assume(__isGlobal(c.claim));
+    __builtin_assume(__isGlobal(c.vote)); __builtin_assume(__isGlobal(c.loc));
+    return c;
+}
+
+template <class SH>
+__device__ __forceinline__ void fast_flips(SH& sh) {
+    Ctx c = fast_view(sh.ctx);
+    const int tid = threadIdx.x;
+    const int* q = sh.ctx.queue;
+    int buf = sh.ctx.queue == sh.queue[0];      // the buffer the next queue goes to
+    int nq = (int)sh.count, sub = 0, turn = 0, flips = 0;
+    const int budget = sh.budget;
+    int carried = sh.ctx.carry_n;               // leading entries carried over from the previous round
+    if (tid == 0) { sh.tally[0][0] = 0; sh.tally[0][1] = 0; }
+    fast_sync<SH::kCap>();
+    do {
+        int* tally = sh.tally[turn];
+        int* qn = sh.queue[buf];
+        turn = turn == 2 ? 0 : turn + 1;
+        if (tid == 0) { sh.tally[turn][0] = 0; sh.tally[turn][1] = 0; }
+        // check
+        int qe = 0;
+        int2 cd = make_int2(-1, -1);
+        if (tid < nq) {
+            qe = q[tid];
+            cd = flip_candidate(c, qe, tid < carried);
+            if (cd.x >= 0) claim_pair(c, cd);
+        }
+        fast_sync<SH::kCap>();
+        // flip
+        const int t = cd.x >> 2, n = cd.y >> 2;
+        FlipRows r;
+        bool won = false;
+        if (cd.x >= 0) {
+            const unsigned long long ck = claim_key(c, cd.x);
+            const unsigned long long c0 = ld_l2(&c.claim[t]), c1 = ld_l2(&c.claim[n]);
+            won = c0 == ck && c1 == ck;
+            if (won) {
+                r = do_flip(c, t, cd.x & 3, n, cd.y & 3, tri_v(c, t), tri_a(c, t), tri_v(c, n), tri_a(c, n));
+                int* qp = qn + 2 * atomicAdd(&tally[0], 1);
+                qp[0] = qentry(t, 5);
+                qp[1] = qentry(n, 3);
+            }
+        }
+        fast_sync<SH::kCap>();
+        // fix: the flip's outer edges; a loser that nobody flipped goes back
+        const int nflip = tally[0];
+        if (won) {
+            const int4 none = make_int4(-1, -1, -1, -1);
+            const int2 nil = make_int2(-1, -1);
+            const int o0 = r.ta.x, o2 = r.ta.z, u0 = r.na.x, u1 = r.na.y;     // old outer neighbours
+            const int4 m0 = o0 >= 0 ? tri_v(c, o0 >> 2) : none, m2 = o2 >= 0 ? tri_v(c, o2 >> 2) : none;
+            const int4 g0 = u0 >= 0 ? tri_v(c, u0 >> 2) : none, g1 = u1 >= 0 ? tri_v(c, u1 >> 2) : none;
+            const int2 p0 = o0 >= 0 ? partner_slots(c, o0 >> 2) : nil, p2 = o2 >= 0 ? partner_slots(c, o2 >> 2) : nil;
+            const int2 q0 = u0 >= 0 ? partner_slots(c, u0 >> 2) : nil, q1 = u1 >= 0 ? partner_slots(c, u1 >> 2) : nil;
+            resolve_flip_loaded(c, t, r.tv, 0, o0, m0, p0);
+            resolve_flip_loaded(c, t, r.tv, 2, o2, m2, p2);
+            resolve_flip_loaded(c, n, r.nv, 0, u0, g0, q0);
+            resolve_flip_loaded(c, n, r.nv, 1, u1, g1, q1);
+        } else if (cd.x >= 0 && flip_stamp(tri_v(c, t).w) != (int)c.sr) {
+            qn[2 * nflip + atomicAdd(&tally[1], 1)] = qe;
+        }
+        fast_sync<SH::kCap>();
+        nq = 2 * nflip + tally[1];
+        flips += nflip;
+        c.sr++;
+        ++sub;
+        carried = 0;
+        q = qn;
+        buf ^= 1;
+    } while (nq > 0 && nq <= SH::kCap && sub < budget);
+    if (tid == 0) { sh.n_queue = nq; sh.subrounds = sub; sh.flips = flips; }
+}
+
+template <class SH>
+__device__ __forceinline__ void fast_round(SH& sh) {
+    const Ctx c = fast_view(sh.ctx);
+    const int tid = threadIdx.x;
+    if (tid == 0) { sh.n_alive = 0; sh.n_won = 0; sh.n_next = 0; sh.n_queue = 0; }
+    const int q = tid < (int)sh.count ? sh.ctx.act[tid] : -1;
+    int t = q >= 0 ? c.loc[q] : -1, e = -1;
+    if (t >= 0) {
+        t = relocate(c, q, t, c.P[q], &e);
+        if (t >= 0) cast_votes(c, q, t, e);
+    }
+    fast_sync<SH::kCap>();
+    int code = -1;
+    if (t >= 0) {
+        const unsigned long long key = vote_key(c, q);
+        if (ld_l2(&c.vote[t]) == key) code = split_rows(c, q, t, e, key);
+    }
+    // survivors, by warp
+    const unsigned alive = __ballot_sync(0xffffffffu, t >= 0), next = __ballot_sync(0xffffffffu, t >= 0 && code < 0);
+    int at = 0;
+    if ((tid & 31) == 0 && alive) {
+        atomicAdd(&sh.n_alive, __popc(alive));
+        if (next) at = atomicAdd(&sh.n_next, __popc(next));
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if ((next >> (tid & 31)) & 1) sh.ctx.act_next[at + __popc(next & ((1u << (tid & 31)) - 1u))] = q;
+    fast_sync<SH::kCap>();
+    if (code >= 0) {
+        int4 qe;
+        const int n = fix_winner(c, make_int2(q * 8 + code, t), qe);
+        int* qn = sh.queue[0] + atomicAdd(&sh.n_queue, n);
+        qn[0] = qe.x; qn[1] = qe.y; qn[2] = qe.z;
+        if (n == 4) qn[3] = qe.w;
+    }
+}
+
+// The fields of the published context that a single-block phase's items
+// use, for the phases of every round and sub-round: loaded once, and known to
+// be in device memory except for the lists and the counters.
+__device__ __forceinline__ Ctx items_view(const Ctx& p, int k) {
+    Ctx c{};
+    c.cnt = p.cnt; c.eslot = p.eslot; c.round = p.round; c.tri = p.tri;
+    __builtin_assume(__isGlobal(c.tri));
+    if (k == K_FLIP_CHECK || k == K_FLIP_DO || k == K_FLIP_FIX) {
+        c.sr = p.sr; c.cand = p.cand;
+        if (k != K_FLIP_FIX) { c.claim = p.claim; __builtin_assume(__isGlobal(c.claim)); }
+        if (k != K_FLIP_DO) c.queue = p.queue;
+        if (k == K_FLIP_CHECK) { c.carry_n = p.carry_n; c.P = p.P; __builtin_assume(__isGlobal(c.P)); }
+        else c.queue_next = p.queue_next;
+        if (k == K_FLIP_DO) c.base_flip = p.base_flip;
+        if (k == K_FLIP_FIX) { c.list_n = p.list_n; c.base_q = p.base_q; }
+    } else if (k == K_FIX) {
+        c.winners = p.winners; c.queue_next = p.queue_next; c.base_q = p.base_q;
+    } else {        // K_RELOC_VOTE, K_SPLIT
+        c.act = p.act; c.loc = p.loc; c.pedge = p.pedge; c.vote = p.vote;
+        __builtin_assume(__isGlobal(c.loc)); __builtin_assume(__isGlobal(c.pedge)); __builtin_assume(__isGlobal(c.vote));
+        if (k == K_SPLIT) { c.winners = p.winners; c.base_win = p.base_win; }
+        else { c.P = p.P; __builtin_assume(__isGlobal(c.P)); c.act_next = p.act_next; c.base_act = p.base_act; }
+    }
+    return c;
+}
+
+template <int K, class SH>
+__device__ __forceinline__ void round_items(const SH& sh) {
+    const Ctx c = items_view(sh.ctx, K);
+    const int count = (int)sh.count, stride = blockDim.x - 32;
+    for (int i = threadIdx.x; i < count; i += stride) dispatch(K, c, i);
+}
+
+// A worker's share of a published single-block phase or command.
+template <class SH>
+__device__ __forceinline__ void block_items(SH& sh) {
+    switch (const int k = sh.kind) {
+    case kFastFlips: if (threadIdx.x < SH::kCap) fast_flips(sh); break;
+    case kFastRound: if (threadIdx.x < SH::kCap) fast_round(sh); break;
+    case K_FLIP_CHECK: round_items<K_FLIP_CHECK>(sh); break;
+    case K_FLIP_DO: round_items<K_FLIP_DO>(sh); break;
+    case K_FLIP_FIX: round_items<K_FLIP_FIX>(sh); break;
+    case K_RELOC_VOTE: round_items<K_RELOC_VOTE>(sh); break;
+    case K_SPLIT: round_items<K_SPLIT>(sh); break;
+    case K_FIX: round_items<K_FIX>(sh); break;
+    default: {
+        const long long count = sh.count, stride = blockDim.x - 32;
+        for (long long i = threadIdx.x; i < count; i += stride) dispatch(k, sh.ctx, (int)i);
+    }
+    }
+}
+
+// ---------------------------------------------------------------- teams
+
+// A worker's items of a team's phase.  W: queue entries per thread and trip
+// in the flip check and fix.
+template <int W>
+struct TeamItems {
+    int& work;      // the block's next chunk, in shared memory
+    unsigned rank, size;    // of the block in its team, of the team
+
+    // The phases that run once or a few times per solve: a plain
+    // team-stride loop.
+    __device__ void other(int k, const Ctx& c, long long count) const {
+        const unsigned workers = blockDim.x - 32;
+        const long long stride = (long long)size * workers;
+        long long i = (long long)rank * workers + threadIdx.x;
+        for (; i < count; i += stride) dispatch(k, c, (int)i);
+    }
+    // Items of a phase in chunks of one warp's worth, chunk j of block b
+    // being chunk b + j * blocks of the phase (the grid-stride interleave);
+    // the block's warps take its chunks in turn from a shared-memory
+    // counter, so a warp that finishes early takes more (28.45 -> 28.03 ms
+    // on the headline solve, for the rounds' and sub-rounds' phases).
+    __device__ int take_chunk() const {
+        int j = 0;
+        if ((threadIdx.x & 31) == 0) j = atomicAdd(&work, 1);
+        return __shfl_sync(0xffffffffu, j, 0);
+    }
+    // The flip passes' chunk loop: each lane's two items of the next chunk
+    // have their first word (queue entry or candidate) loaded while the
+    // current chunk runs.
+    // The flip pass two chunks ahead: chunk j+2's candidates are loaded, and
+    // the claims chunk j+1's candidates name are prefetched into L2, while
+    // chunk j runs.  (The same second stage in the check and the fix, an L2
+    // prefetch of the rows their next chunk names, made them slower.)
+    template <int P, int E>
+    __device__ void pipelined(const Ctx& c, long long count, int j) const {
+        constexpr bool kTwoAhead = P == FP_DO;
+        const int lane = threadIdx.x & 31;
+        auto chunk_at = [&](int jj) { return ((long long)rank + (long long)jj * size) * (32 * E); };
+        auto load = [&](long long b, int (&k)[E], int2 (&f)[E]) {
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                k[u] = b + lane + 32 * u < count ? (int)(b + lane + 32 * u) : -1;
+                f[u] = flip_first(c, P, k[u]);
+            }
+        };
+        int ks[E], ns[E];
+        int2 f[E], g[E];
+        long long base = chunk_at(j), next = 0;
+        load(base, ks, f);
+        if (kTwoAhead) {
+            j = take_chunk();
+            next = chunk_at(j);
+            load(next, ns, g);
+        }
+        while (base < count) {
+            j = take_chunk();
+            const long long at = chunk_at(j);
+            int ms[E];
+            int2 h[E];
+            load(at, ms, h);
+            if (kTwoAhead) {
+#pragma unroll
+                for (int u = 0; u < E; ++u)
+                    if (ns[u] >= 0 && g[u].x >= 0) prefetch_l2(&c.claim[g[u].x >> 2], &c.claim[g[u].y >> 2]);
+            }
+            if (ks[0] >= 0) {
+                if (P == FP_CHECK) flip_check_multi_f<E>(c, ks, f);
+                else if (P == FP_DO) flip_do_multi_f<E>(c, ks, f);
+                else flip_fix_multi_f<E>(c, ks, f);
+            }
+            base = kTwoAhead ? next : at;
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                ks[u] = kTwoAhead ? ns[u] : ms[u];
+                f[u] = kTwoAhead ? g[u] : h[u];
+                if (kTwoAhead) { ns[u] = ms[u]; g[u] = h[u]; }
+            }
+            if (kTwoAhead) next = at;
+        }
+    }
+    __device__ static void prefetch_l2(const void* a, const void* b) {
+        asm volatile("prefetch.global.L2 [%0];" :: "l"(a));
+        asm volatile("prefetch.global.L2 [%0];" :: "l"(b));
+    }
+    template <int K>
+    __device__ void round(const Ctx& c, long long count) const {
+        constexpr int chunk = 32 * (K == K_FLIP_DO ? 2 : (K == K_FLIP_CHECK || K == K_FLIP_FIX) ? W : 1);
+        const int lane = threadIdx.x & 31;
+        auto chunk_at = [&](int jj) { return ((long long)rank + (long long)jj * size) * chunk; };
+        int j = take_chunk();
+        long long base = chunk_at(j);
+        if (base >= count) return;          // fewer chunks than warps
+        if constexpr (K == K_FLIP_CHECK) {
+            pipelined<FP_CHECK, W>(c, count, j);
+        } else if constexpr (K == K_FLIP_DO) {
+            pipelined<FP_DO, 2>(c, count, j);
+        } else if constexpr (K == K_FLIP_FIX) {
+            pipelined<FP_FIX, W>(c, count, j);
+        } else if constexpr (K == K_FIX) {
+            int2 w = base + lane < count ? c.winners[base + lane] : make_int2(-1, -1);
+            while (base < count) {
+                j = take_chunk();
+                const long long nb = chunk_at(j);
+                const int2 nw = nb + lane < count ? c.winners[nb + lane] : make_int2(-1, -1);
+                if (w.x >= 0) body_fix_f(c, w);
+                base = nb; w = nw;
+            }
+        } else {
+            // relocation and split, two chunks ahead: the active points of
+            // chunk j+2 and the locations (and, for the relocation,
+            // coordinates) of chunk j+1's points are loaded while chunk j
+            // runs (each point's item is the only one that writes its
+            // location)
+            constexpr bool rv = K == K_RELOC_VOTE;
+            int q = base + lane < count ? c.act[base + lane] : -1;
+            int t = q >= 0 ? c.loc[q] : -1;
+            int2 p = (rv && t >= 0) ? c.P[q] : make_int2(0, 0);
+            j = take_chunk();
+            long long nb = chunk_at(j);
+            int nq = nb + lane < count ? c.act[nb + lane] : -1;
+            while (base < count) {
+                j = take_chunk();
+                const long long nnb = chunk_at(j);
+                const int nnq = nnb + lane < count ? c.act[nnb + lane] : -1;
+                const int nt = nq >= 0 ? c.loc[nq] : -1;
+                const int2 np = (rv && nq >= 0) ? c.P[nq] : make_int2(0, 0);
+                if (q >= 0) {
+                    if (rv) body_reloc_vote_qt(c, q, t, p);
+                    else body_split_qt(c, q, t);
+                }
+                base = nb; q = nq; t = nt; p = np; nb = nnb; nq = nnq;
+            }
+        }
+    }
+};
+
+// Cluster barrier, by all threads of its blocks; what they wrote before it
+// is visible to all after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+
+// Driver of one block of a team (every block runs the same control flow on
+// the same values).
+template <bool kCluster, class SH>
+struct TeamExec {
     static constexpr bool kCanNarrow = true;
     Counters* cnt;
-    unsigned nblocks;
+    unsigned rank, size;                     // of the block in its team, of the team
+    SH* sh;
+    unsigned spin_limit = 1u << 24;          // polls before a grid barrier wait gives up
+    bool prof = false;                       // record the phase profile and balance (a launch constant)
+    // Snapshot of the head of Counters (status, error words, list cursors),
+    // word k in lane k, read right after each barrier.
+    unsigned long long snap = 0;
+
     __device__ int narrow_flips(Ctx& c, Driver& D, long long& nq);
     __device__ int narrow_rounds(Ctx& c, Driver& D, long long nact);
 
-    // Snapshot of the head of Counters (status, error words, list cursors)
-    // taken by thread 0 right after each grid barrier: the driver's reads of
-    // these values come from shared memory instead of every thread reading
-    // the same L2 line.
-    static constexpr int kSnapWords = 12;   // 96 bytes: status..cur_scr
-    unsigned long long* snap;                // shared memory, kSnapWords entries
-    unsigned spin_limit = 1u << 24;          // polls before a barrier wait gives up
-    int* work = nullptr;                     // shared memory: the block's next item (dynamic phases)
-    const Ctx* param = nullptr;              // the launch's context, in kernel parameter space
-    bool prof = false;                       // record the phase profile and balance (a launch constant)
-
     __device__ void take_snapshot() {
-        volatile unsigned long long* src = reinterpret_cast<volatile unsigned long long*>(cnt);
-        for (int k = 0; k < kSnapWords; ++k) snap[k] = src[k];
+        const int lane = threadIdx.x & 31;
+        snap = lane < kSnapWords ? reinterpret_cast<volatile unsigned long long*>(cnt)[lane] : 0;
     }
 
     // Grid barrier on one counter whose top bit flips once per barrier:
@@ -74,76 +624,68 @@ struct GridExec {
     // 0 (the solve clears its counters).  Every wait is bounded: after
     // spin_limit polls (2^24, about a second, in a solve) the block records
     // ST_BARRIER and stops waiting, and once that bit is set no block waits
-    // or works any more, so the kernel always ends.
-    __device__ void barrier() { barrier_timed(-1, 0, 0); }
-    // The barrier ending a phase: with k >= 0, thread 0 first records the
-    // block's work time (cycles since t0) for the phase balance.
-    __device__ void barrier_timed(int k, long long t0, int slot) {
-        __syncthreads();
-        if (threadIdx.x == 0 && k >= 0) {
-            unsigned long long w = (unsigned long long)(clock64() - t0);
+    // or works any more, so the kernel always ends.  The driver warp alone
+    // takes part: the block's workers have reported to it (kBarDone) and
+    // wait for the next phase.
+    // In a cluster the hardware's barrier, which the workers take part in as
+    // well (they go to it from their items, or are sent by kTeamSync).
+    __device__ void barrier() {
+        if constexpr (kCluster) {
+            publish(*sh, kTeamSync, sh->ctx, 0, false);
+            block_sync(kBarWork);
+            join();
+        } else {
+            grid_barrier();
+            take_snapshot();
+        }
+    }
+    __device__ void join() {
+        __syncwarp();
+        cluster_sync();
+        take_snapshot();
+    }
+    __device__ void grid_barrier() {
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) {
+            volatile unsigned* vcount = &cnt->bar_count;
+            volatile int* vst = &cnt->status;
+            if (!(*vst & ST_BARRIER)) {
+                const unsigned add = rank == 0 ? 0x80000000u - (size - 1) : 1u;
+                __threadfence();
+                const unsigned old = atomicAdd(&cnt->bar_count, add);
+                // the arrival that completes the count flips the top bit itself
+                const bool last = (((old + add) ^ old) & 0x80000000u) != 0;
+                unsigned spins = 0;
+                while (!last && ((old ^ *vcount) & 0x80000000u) == 0) {
+                    if (++spins > spin_limit) { atomicOr(&cnt->status, ST_BARRIER); break; }
+                    if (*vst & ST_BARRIER) break;
+                    __nanosleep(64);
+                }
+            }
+            __threadfence();
+        }
+        // the snapshot words read by twelve lanes at once, after lane 0 has
+        // seen the barrier open (3.20 -> 2.90 us per barrier against one
+        // lane reading all of them)
+        __syncwarp();
+    }
+    __device__ void phase(int k, const Ctx& c, long long count) {
+        const bool lead = (threadIdx.x & 31) == 0;
+        const long long t0 = prof ? clock64() : 0;
+        const int slot = c.eslot & 1;
+        if (kCluster || !(word(&cnt->status) & ST_BARRIER)) {
+            publish(*sh, k, c, count, false);
+            block_sync(kBarWork);
+            if (!kCluster) block_sync(kBarDone);
+        }
+        if (prof && lead) {     // the block's work time, for the phase balance
+            const unsigned long long w = (unsigned long long)(clock64() - t0);
             atomicMax(&cnt->wcur_max[slot], w);
             atomicAdd(&cnt->wcur_sum[slot], w);
         }
-        if (threadIdx.x < 32) {
-            if (threadIdx.x == 0) {
-                volatile unsigned* vcount = &cnt->bar_count;
-                volatile int* vst = &cnt->status;
-                if (!(*vst & ST_BARRIER)) {
-                    const unsigned add = blockIdx.x == 0 ? 0x80000000u - (nblocks - 1) : 1u;
-                    __threadfence();
-                    const unsigned old = atomicAdd(&cnt->bar_count, add);
-                    // the arrival that completes the count flips the top bit itself
-                    const bool last = (((old + add) ^ old) & 0x80000000u) != 0;
-                    unsigned spins = 0;
-                    while (!last && ((old ^ *vcount) & 0x80000000u) == 0) {
-                        if (++spins > spin_limit) { atomicOr(&cnt->status, ST_BARRIER); break; }
-                        if (*vst & ST_BARRIER) break;
-                        __nanosleep(64);
-                    }
-                }
-                __threadfence();
-            }
-            // the snapshot words read by the first lanes of warp 0 at once,
-            // after lane 0 has seen the barrier open (3.20 -> 2.90 us per
-            // barrier against one lane reading all of them)
-            __syncwarp();
-            if (threadIdx.x < kSnapWords)
-                snap[threadIdx.x] = reinterpret_cast<volatile unsigned long long*>(cnt)[threadIdx.x];
-        }
-        __syncthreads();
-    }
-    __device__ void phase(int k, const Ctx& cd, long long count) {
-        const Ctx c = phase_view(*param, cd);
-        long long t0 = threadIdx.x == 0 ? clock64() : 0;
-        // the rounds' and flip sub-rounds' phases take their items in warp
-        // chunks (28.45 -> 28.03 ms on the headline solve); the others, one
-        // or a few runs per solve, keep the plain grid-stride loop
-        if (!(word(&cnt->status) & ST_BARRIER) && work &&
-            (k == K_FLIP_CHECK || k == K_FLIP_DO || k == K_FLIP_FIX || k == K_RELOC_VOTE || k == K_SPLIT ||
-             k == K_FIX)) {
-            dynamic_items(k, c, count);
-        } else if (!(word(&cnt->status) & ST_BARRIER)) {
-            long long stride = (long long)gridDim.x * blockDim.x;
-            long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-            // latency-bound passes: two items per thread and trip (i, i + stride)
-            if (k == K_FLIP_CHECK) {
-                for (; i < count; i += 2 * stride)
-                    body_flip_check_pair(c, (int)i, i + stride < count ? (int)(i + stride) : -1);
-            } else if (k == K_FLIP_DO) {
-                for (; i < count; i += 2 * stride)
-                    body_flip_do_pair(c, (int)i, i + stride < count ? (int)(i + stride) : -1);
-            } else if (k == K_FLIP_FIX) {
-                for (; i < count; i += 2 * stride)
-                    body_flip_fix_pair(c, (int)i, i + stride < count ? (int)(i + stride) : -1);
-            } else {
-                for (; i < count; i += stride) dispatch(k, c, (int)i);
-            }
-        }
-        const int slot = c.eslot & 1;
-        const bool timer = prof && blockIdx.x == 0 && threadIdx.x == 0;
-        barrier_timed(prof && k < kMaxPhaseKinds ? k : -1, t0, slot);
-        if (timer && k < kMaxPhaseKinds) {   // phase time incl. the barrier, as block 0 sees it
+        if constexpr (kCluster) join();
+        else barrier();
+        if (prof && lead && rank == 0 && k < kMaxPhaseKinds) {   // phase time incl. the barrier, as block 0 sees it
             cnt->phase_cyc[k] += clock64() - t0;
             cnt->phase_cnt[k] += 1;
             // every block added this run's work time before it arrived; no
@@ -155,150 +697,19 @@ struct GridExec {
             cnt->wcur_sum[slot] = 0;
         }
     }
-    // Items of a phase in chunks of one warp's worth, chunk j of block b
-    // being chunk b + j * blocks of the phase (the grid-stride interleave);
-    // the block's warps take its chunks in turn from a shared-memory
-    // counter, so a warp that finishes early takes more.
-    __device__ int take_chunk() {
-        int j = 0;
-        if ((threadIdx.x & 31) == 0) j = atomicAdd(work, 1);
-        return __shfl_sync(0xffffffffu, j, 0);
-    }
-    // The flip passes' chunk loop: each lane's two items of the next chunk
-    // have their first word (queue entry or candidate) loaded while the
-    // current chunk runs.
-    // The flip pass two chunks ahead: chunk j+2's candidates are loaded, and
-    // the claims chunk j+1's candidates name are prefetched into L2, while
-    // chunk j runs.  (The same second stage in the check and the fix, an L2
-    // prefetch of the rows their next chunk names, made them slower.)
-    __device__ void flip_do_pipelined(const Ctx& c, long long count, int j) {
-        const int lane = threadIdx.x & 31;
-        auto chunk_at = [&](int jj) { return ((long long)blockIdx.x + (long long)jj * gridDim.x) * 64; };
-        auto item = [&](long long b, int o) { return b + lane + o < count ? (int)(b + lane + o) : -1; };
-        long long base = chunk_at(j);
-        int k0 = item(base, 0), k1 = item(base, 32);
-        int2 f0 = flip_first(c, FP_DO, k0), f1 = flip_first(c, FP_DO, k1);
-        j = take_chunk();
-        long long nb = chunk_at(j);
-        int n0 = item(nb, 0), n1 = item(nb, 32);
-        int2 g0 = flip_first(c, FP_DO, n0), g1 = flip_first(c, FP_DO, n1);
-        while (base < count) {
-            j = take_chunk();
-            const long long nnb = chunk_at(j);
-            const int m0 = item(nnb, 0), m1 = item(nnb, 32);
-            const int2 h0 = flip_first(c, FP_DO, m0), h1 = flip_first(c, FP_DO, m1);
-            if (n0 >= 0 && g0.x >= 0) prefetch_l2(&c.claim[g0.x >> 2], &c.claim[g0.y >> 2]);
-            if (n1 >= 0 && g1.x >= 0) prefetch_l2(&c.claim[g1.x >> 2], &c.claim[g1.y >> 2]);
-            if (k0 >= 0) {
-                const int ks[2] = {k0, k1};
-                const int2 f[2] = {f0, f1};
-                body_flip_do_pair_f(c, ks, f);
-            }
-            base = nb; k0 = n0; k1 = n1; f0 = g0; f1 = g1;
-            nb = nnb; n0 = m0; n1 = m1; g0 = h0; g1 = h1;
-        }
-    }
-    __device__ static void prefetch_l2(const void* a, const void* b) {
-        asm volatile("prefetch.global.L2 [%0];" :: "l"(a));
-        asm volatile("prefetch.global.L2 [%0];" :: "l"(b));
-    }
-    template <int P>
-    __device__ void pipelined(const Ctx& c, long long count, int j) {
-        const int lane = threadIdx.x & 31;
-        long long base = ((long long)blockIdx.x + (long long)j * gridDim.x) * 64;
-        int k0 = base + lane < count ? (int)(base + lane) : -1;
-        int k1 = base + lane + 32 < count ? (int)(base + lane + 32) : -1;
-        int2 f0 = flip_first(c, P, k0), f1 = flip_first(c, P, k1);
-        while (base < count) {
-            j = take_chunk();
-            const long long nb = ((long long)blockIdx.x + (long long)j * gridDim.x) * 64;
-            const int n0 = nb + lane < count ? (int)(nb + lane) : -1;
-            const int n1 = nb + lane + 32 < count ? (int)(nb + lane + 32) : -1;
-            const int2 g0 = flip_first(c, P, n0), g1 = flip_first(c, P, n1);
-            if (k0 >= 0) {
-                const int ks[2] = {k0, k1};
-                const int2 f[2] = {f0, f1};
-                if (P == FP_CHECK) flip_check_multi_f<2>(c, ks, f);
-                else if (P == FP_DO) body_flip_do_pair_f(c, ks, f);
-                else body_flip_fix_pair_f(c, ks, f);
-            }
-            base = nb; k0 = n0; k1 = n1; f0 = g0; f1 = g1;
-        }
-    }
-    __device__ void dynamic_items(int k, const Ctx& c, long long count) {
-        if (threadIdx.x == 0) *work = 0;
-        __syncthreads();
-        const bool pair = k == K_FLIP_CHECK || k == K_FLIP_DO || k == K_FLIP_FIX;
-        const long long chunk = pair ? 64 : 32;
-        const int lane = threadIdx.x & 31;
-        int j = take_chunk();
-        if (pair) {
-            if (k == K_FLIP_CHECK) pipelined<FP_CHECK>(c, count, j);
-            else if (k == K_FLIP_DO) flip_do_pipelined(c, count, j);
-            else pipelined<FP_FIX>(c, count, j);
-            return;
-        }
-        if (k == K_RELOC_VOTE || k == K_SPLIT) {
-            // two chunks ahead: the active points of chunk j+2 and the
-            // locations (and, for the relocation, coordinates) of chunk j+1's
-            // points are loaded while chunk j runs (each point's item is the
-            // only one that writes its location)
-            const bool rv = k == K_RELOC_VOTE;
-            long long base = ((long long)blockIdx.x + (long long)j * gridDim.x) * chunk;
-            int q = base + lane < count ? c.act[base + lane] : -1;
-            int t = q >= 0 ? c.loc[q] : -1;
-            int2 p = (rv && t >= 0) ? c.P[q] : make_int2(0, 0);
-            j = take_chunk();
-            long long nb = ((long long)blockIdx.x + (long long)j * gridDim.x) * chunk;
-            int nq = nb + lane < count ? c.act[nb + lane] : -1;
-            while (base < count) {
-                j = take_chunk();
-                const long long nnb = ((long long)blockIdx.x + (long long)j * gridDim.x) * chunk;
-                const int nnq = nnb + lane < count ? c.act[nnb + lane] : -1;
-                const int nt = nq >= 0 ? c.loc[nq] : -1;
-                const int2 np = (rv && nq >= 0) ? c.P[nq] : make_int2(0, 0);
-                if (q >= 0) {
-                    if (rv) body_reloc_vote_qt(c, q, t, p);
-                    else body_split_qt(c, q, t);
-                }
-                base = nb; q = nq; t = nt; p = np; nb = nnb; nq = nnq;
-            }
-            return;
-        }
-        if (k == K_FIX) {
-            long long base = ((long long)blockIdx.x + (long long)j * gridDim.x) * chunk;
-            int2 w = base + lane < count ? c.winners[base + lane] : make_int2(-1, -1);
-            while (base < count) {
-                j = take_chunk();
-                const long long nb = ((long long)blockIdx.x + (long long)j * gridDim.x) * chunk;
-                const int2 nw = nb + lane < count ? c.winners[nb + lane] : make_int2(-1, -1);
-                if (w.x >= 0) body_fix_f(c, w);
-                base = nb; w = nw;
-            }
-            return;
-        }
-        for (;;) {
-            const long long base = ((long long)blockIdx.x + (long long)j * gridDim.x) * chunk;
-            if (base >= count) break;
-            const long long i0 = base + lane;
-            if (i0 < count) dispatch(k, c, (int)i0);
-            j = take_chunk();
-        }
-    }
-    // Values read after a barrier come from the block's snapshot.
+    // Values read after a barrier come from the snapshot.
     __device__ unsigned long long cursor(unsigned long long* p) {
-        size_t off = (size_t)((char*)p - (char*)cnt);
-        if (off + 8 <= kSnapWords * 8) return *reinterpret_cast<unsigned long long*>((char*)snap + off);
-        return *(volatile unsigned long long*)p;
+        const int at = (int)((char*)p - (char*)cnt);
+        return __shfl_sync(0xffffffffu, snap, at >> 3);
     }
     __device__ int word(int* p) {
-        size_t off = (size_t)((char*)p - (char*)cnt);
-        if (off + 4 <= kSnapWords * 8) return *reinterpret_cast<int*>((char*)snap + off);
-        return *(volatile int*)p;
+        const int at = (int)((char*)p - (char*)cnt);
+        const unsigned long long w = __shfl_sync(0xffffffffu, snap, at >> 3);
+        return (int)(at & 4 ? w >> 32 : w);
     }
     __device__ void finish(const Ctx&, long long rounds, long long subrounds, long long crounds, int rc) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            cnt->grid_blocks = nblocks;
+        if (rank == 0 && (threadIdx.x & 31) == 0) {
+            cnt->grid_blocks = size;
             cnt->rounds = rounds;
             cnt->flip_subrounds = subrounds;
             cnt->constraint_rounds = crounds;
@@ -307,62 +718,48 @@ struct GridExec {
     }
 };
 
-// Executor of one block: a phase is a block-stride loop and a block barrier.
-// Used by block 0 for the short tails while the other blocks wait, and by
-// every block of the batched kernel (kView: the items see phase_view of
-// the block's context in shared memory).
-template <bool kView>
-struct BlockExecT {
-    static constexpr bool kCanNarrow = false;
-    Counters* cnt;
-    const Ctx* base = nullptr;
-    __device__ void phase(int k, const Ctx& cd, long long count) {
-        if constexpr (kView) items(k, phase_view(*base, cd), count);
-        else items(k, cd, count);
-        __syncthreads();
-    }
-    __device__ void items(int k, const Ctx& c, long long count) {
-        const long long stride = blockDim.x;
-        long long i = threadIdx.x;
-        // the latency-bound flip passes: two items per thread and trip, as
-        // on the grid, so a queue of up to two blocks' worth is one trip
-#ifndef GCDT_BLOCK_PAIRS
-#define GCDT_BLOCK_PAIRS 1
-#endif
-        if (!GCDT_BLOCK_PAIRS) {
-            for (; i < count; i += stride) dispatch(k, c, (int)i);
-        } else if (k == K_FLIP_CHECK) {
-            for (; i < count; i += 2 * stride)
-                body_flip_check_pair(c, (int)i, i + stride < count ? (int)(i + stride) : -1);
-        } else if (k == K_FLIP_DO) {
-            for (; i < count; i += 2 * stride)
-                body_flip_do_pair(c, (int)i, i + stride < count ? (int)(i + stride) : -1);
-        } else if (k == K_FLIP_FIX) {
-            for (; i < count; i += 2 * stride)
-                body_flip_fix_pair(c, (int)i, i + stride < count ? (int)(i + stride) : -1);
-        } else {
-            for (; i < count; i += stride) dispatch(k, c, (int)i);
+constexpr int kStageCap = 512;
+using StageShared = BlockShared<kStageCap>;
+static_assert(kStageCap <= 32 * kStageWorkers, "the fast commands take one worker thread per entry");
+using GridExec = TeamExec<false, StageShared>;
+
+// The body of a team block's worker warps.  view.items<K>() and view.other()
+// give the context of a team phase's items.
+template <bool kCluster, int W, class SH, class View>
+__device__ __forceinline__ void team_worker(SH& sh, unsigned rank, unsigned size, const View& view) {
+    const TeamItems<W> items{sh.work, rank, size};
+    for (;;) {
+        block_sync(kBarWork);
+        const int k = sh.kind;
+        if (k == kExit) return;
+        if (sh.single) {
+            block_items(sh);
+            block_sync(kBarDone);
+            continue;
         }
-    }
-    __device__ unsigned long long cursor(unsigned long long* p) { return *(volatile unsigned long long*)p; }
-    __device__ int word(int* p) { return *(volatile int*)p; }
-    __device__ void finish(const Ctx&, long long rounds, long long subrounds, long long crounds, int rc) {
-        if (threadIdx.x == 0) {
-            cnt->rounds = rounds;
-            cnt->flip_subrounds = subrounds;
-            cnt->constraint_rounds = crounds;
-            if (rc) atomicOr(&cnt->status, rc);
+        switch (k) {
+        case kTeamSync: break;
+        case K_FLIP_CHECK: items.template round<K_FLIP_CHECK>(view.template items<K_FLIP_CHECK>(), sh.count); break;
+        case K_FLIP_DO: items.template round<K_FLIP_DO>(view.template items<K_FLIP_DO>(), sh.count); break;
+        case K_FLIP_FIX: items.template round<K_FLIP_FIX>(view.template items<K_FLIP_FIX>(), sh.count); break;
+        case K_RELOC_VOTE: items.template round<K_RELOC_VOTE>(view.template items<K_RELOC_VOTE>(), sh.count); break;
+        case K_SPLIT: items.template round<K_SPLIT>(view.template items<K_SPLIT>(), sh.count); break;
+        case K_FIX: items.template round<K_FIX>(view.template items<K_FIX>(), sh.count); break;
+        default: items.other(k, view.other(), sh.count); break;
         }
+        __syncwarp();
+        if (kCluster) cluster_sync();
+        else block_sync(kBarDone);
     }
-    __device__ int narrow_flips(Ctx&, Driver&, long long&) { return ST_INTERNAL; }
-    __device__ int narrow_rounds(Ctx&, Driver&, long long) { return ST_INTERNAL; }
-};
-using BlockExec = BlockExecT<false>;
+}
 
 static_assert(sizeof(Driver) <= sizeof(((Counters*)0)->handoff), "driver state fits the hand-off area");
 static_assert(sizeof(Driver) % 8 == 0, "driver state is whole 8-byte words");
 
+// The driver state after a single-block tail, and the list cursors, which
+// the tail kept in the block's own counters.
 __device__ inline void store_handoff(Counters* cnt, const Driver& D, long long nq, int rc) {
+    cnt->cur_act = D.e_act; cnt->cur_win = D.e_win; cnt->cur_q = D.e_q; cnt->cur_flip = D.e_flip;
     save_driver(cnt, D);
     cnt->handoff_nq = nq;
     cnt->handoff_rc = rc;
@@ -374,16 +771,20 @@ __device__ inline int load_handoff(Counters* cnt, Driver& D, long long& nq) {
     return *(volatile int*)&cnt->handoff_rc;
 }
 
-__device__ inline int GridExec::narrow_flips(Ctx& c, Driver& D, long long& nq) {
-    const bool timer = prof && blockIdx.x == 0 && threadIdx.x == 0;
+template <bool kCluster, class SH>
+__device__ inline int TeamExec<kCluster, SH>::narrow_flips(Ctx& c, Driver& D, long long& nq) {
+    const bool timer = prof && rank == 0 && (threadIdx.x & 31) == 0;
     long long t0 = timer ? clock64() : 0;
-    if (blockIdx.x == 0) {
-        BlockExec bx{cnt};
+    if (rank == 0) {
+        BlockExecT<SH> bx(*sh, c);
         Driver Db = D;
         Ctx cb = c;
+        cb.cnt = bx.begin(Db);
+        bx.cur_q = Db.qa;
         long long left = nq;
         int rc = flip_loop(bx, cb, Db, left, 4 * (long long)c.narrow_q);
-        if (threadIdx.x == 0) store_handoff(cnt, Db, left, rc);
+        if (rc == 0) bx.store_queue(Db.qa, left);
+        if ((threadIdx.x & 31) == 0) store_handoff(cnt, Db, left, rc);
     }
     barrier();
     int rc = load_handoff(cnt, D, nq);
@@ -391,15 +792,18 @@ __device__ inline int GridExec::narrow_flips(Ctx& c, Driver& D, long long& nq) {
     return rc;
 }
 
-__device__ inline int GridExec::narrow_rounds(Ctx& c, Driver& D, long long nact) {
-    const bool timer = prof && blockIdx.x == 0 && threadIdx.x == 0;
+template <bool kCluster, class SH>
+__device__ inline int TeamExec<kCluster, SH>::narrow_rounds(Ctx& c, Driver& D, long long nact) {
+    const bool timer = prof && rank == 0 && (threadIdx.x & 31) == 0;
     long long t0 = timer ? clock64() : 0;
-    if (blockIdx.x == 0) {
-        BlockExec bx{cnt};
+    if (rank == 0) {
+        BlockExecT<SH> bx(*sh, c);
         Driver Db = D;
         Ctx cb = c;
+        cb.cnt = bx.begin(Db);
+        bx.cur_act = Db.actA;
         int rc = insert_rounds(bx, cb, Db, nact);
-        if (threadIdx.x == 0) store_handoff(cnt, Db, 0, rc);
+        if ((threadIdx.x & 31) == 0) store_handoff(cnt, Db, 0, rc);
     }
     barrier();
     long long dummy;
@@ -407,6 +811,5 @@ __device__ inline int GridExec::narrow_rounds(Ctx& c, Driver& D, long long nact)
     if (timer) { cnt->phase_cyc[K_NARROW_ROUNDS] += clock64() - t0; cnt->phase_cnt[K_NARROW_ROUNDS] += 1; }
     return rc;
 }
-
 
 }  // namespace gcdt

@@ -280,6 +280,15 @@ GCDT_HD int append_slots(unsigned long long* cur, unsigned long long base, int c
 #endif
 }
 
+// A word that other threads' atomics change, read where they act (L2).
+GCDT_HD unsigned long long ld_l2(const unsigned long long* p) {
+#if defined(__CUDA_ARCH__)
+    return __ldcg(p);
+#else
+    return *p;
+#endif
+}
+
 GCDT_HD unsigned long long morton60(int2 p) {
     unsigned long long x = (unsigned)p.x, y = (unsigned)p.y;
     auto spread = [](unsigned long long v) {
@@ -411,8 +420,9 @@ GCDT_HD void body_root(const Ctx& c, int) {
 // randomized insertion order over the spatial sort).
 GCDT_HD void body_level(const Ctx& c, int i) {
     int l = c.nlevels - 1;
-    for (int k = 0; k + 1 < c.nlevels; ++k)
-        if (i % c.stride[k] == 0) { l = k; break; }
+#pragma unroll
+    for (int k = 2; k >= 0; --k)
+        if (k + 1 < c.nlevels && i % c.stride[k] == 0) l = k;
     c.lvl[i] = (unsigned char)l;
 }
 
@@ -493,7 +503,9 @@ GCDT_HD void body_activate(const Ctx& c, int i) {
     } else {
         // start from the nearer of the two previous-level samples around i
         // in curve order (both are vertices already)
-        const int s = c.stride[c.level - 1];
+        // (no index computed at run time: it would keep a grid phase's whole
+        // view of the context in local memory)
+        const int s = c.level == 1 ? c.stride[0] : (c.level == 2 ? c.stride[1] : c.stride[2]);
         int sv = i - i % s;
         const int hi = sv + s;
         const int2 p = c.P[i];
@@ -568,34 +580,51 @@ GCDT_HD int edge_of(const Ctx& c, int t, int2 p) {
     return o0 == 0 ? 0 : (o1 == 0 ? 1 : (o2 == 0 ? 2 : -1));
 }
 
-// Active point q (its location t = loc[q] and coordinates p loaded by the
-// caller): relocate if its triangle changed in the previous round, keep it
-// in the next list, and vote for the triangle(s) it will split.  Winner per
-// triangle = minimum hash32(q): random insertion order per triangle,
-// independent of thread scheduling.
-GCDT_HD void body_reloc_vote_qt(const Ctx& c, int q, int t, int2 p) {
-    if (t < 0) return;                       // inserted last round
-    int e;
-    if (tri_a(c, t).w == (int)c.round - 1) {
-        int nt = walk(c, t, p, 256, &e);
-        if (nt < 0) {
-            nt = locate_from_vertex(c, tri_v(c, t).x, t, p);
-            if (nt < 0) { fail(c, ST_ITER_LIMIT); return; }
-            e = edge_of(c, nt, p);
-        }
-        t = nt;
-        c.loc[q] = t;
-    } else {
-        e = edge_of(c, t, p);
+// Triangle that holds active point q (coordinates p) now, given the one that
+// held it (t): a walk if that triangle changed in the previous round.  *e is
+// the slot of the edge that p lies on, or -1; -1 is returned when the walk's
+// bound ran out.
+GCDT_HD int relocate(const Ctx& c, int q, int t, int2 p, int* e) {
+    if (tri_a(c, t).w != (int)c.round - 1) {
+        *e = edge_of(c, t, p);
+        return t;
     }
-    c.act_next[append_slot(&c.cnt->cur_act, c.base_act)] = q;
-    c.pedge[q] = (signed char)e;
-    unsigned long long key = ((unsigned long long)c.round << 32) | (0xffffffffu - hash32((uint32_t)q));
+    int nt = walk(c, t, p, 256, e);
+    if (nt < 0) {
+        nt = locate_from_vertex(c, tri_v(c, t).x, t, p);
+        if (nt < 0) { fail(c, ST_ITER_LIMIT); return -1; }
+        *e = edge_of(c, nt, p);
+    }
+    c.loc[q] = nt;
+    return nt;
+}
+
+GCDT_HD unsigned long long vote_key(const Ctx& c, int q) {
+    return ((unsigned long long)c.round << 32) | (0xffffffffu - hash32((uint32_t)q));
+}
+
+// Vote for the triangle(s) that point q in triangle t, on its edge e (-1:
+// inside), will split.  Winner per triangle = minimum hash32(q): random
+// insertion order per triangle, independent of thread scheduling.
+GCDT_HD void cast_votes(const Ctx& c, int q, int t, int e) {
+    const unsigned long long key = vote_key(c, q);
     if (c.vote[t] < key) at_max64(&c.vote[t], key);
     if (e >= 0) {
         int n = comp(tri_a(c, t), e) >> 2;
         if (c.vote[n] < key) at_max64(&c.vote[n], key);
     }
+}
+
+// Active point q (its location t = loc[q] and coordinates p loaded by the
+// caller): relocate, keep it in the next list, and vote.
+GCDT_HD void body_reloc_vote_qt(const Ctx& c, int q, int t, int2 p) {
+    if (t < 0) return;                       // inserted last round
+    int e;
+    t = relocate(c, q, t, p, &e);
+    if (t < 0) return;
+    c.act_next[append_slot(&c.cnt->cur_act, c.base_act)] = q;
+    c.pedge[q] = (signed char)e;
+    cast_votes(c, q, t, e);
 }
 GCDT_HD void body_reloc_vote(const Ctx& c, int k) {
     const int q = c.act[k], t = c.loc[q];
@@ -605,8 +634,9 @@ GCDT_HD void body_reloc_vote(const Ctx& c, int k) {
 // Winners split their triangle(s).  Child j of a split triangle is the
 // triangle with vertex j replaced by q; it keeps the old edge j in slot j.
 // Outer adjacency is written as the old neighbour and resolved in body_fix.
-GCDT_HD void split_winner(const Ctx& c, int q, int t, unsigned long long key) {
-    int e = c.pedge[q];
+// Returns the winner's split code (7: inside, else the split edge's slot),
+// or -1 if q lost the triangle across the edge it lies on.
+GCDT_HD int split_rows(const Ctx& c, int q, int t, int e, unsigned long long key) {
     int T1 = 2 + 2 * q, T2 = 3 + 2 * q;
     int4 tv = tri_v(c, t), ta = tri_a(c, t);
     int fl = tv.w;
@@ -626,7 +656,7 @@ GCDT_HD void split_winner(const Ctx& c, int q, int t, unsigned long long key) {
     } else {
         int en = comp(ta, e);
         int n = en >> 2, e2 = en & 3;
-        if (c.vote[n] != key) return;
+        if (ld_l2(&c.vote[n]) != key) return -1;
         int4 nv = tri_v(c, n), na = tri_a(c, n);
         int gl = nv.w;
         // children: A1 = child_{e+1}(t) -> t, A2 = child_{e+2}(t) -> T1,
@@ -656,13 +686,14 @@ GCDT_HD void split_winner(const Ctx& c, int q, int t, unsigned long long key) {
         tri_v(c, B2) = v; tri_a(c, B2) = a;
     }
     c.loc[q] = -1;
-    c.winners[append_slot(&c.cnt->cur_win, c.base_win)] = make_int2(q * 8 + code, t);
+    return code;
 }
 
 GCDT_HD void body_split_qt(const Ctx& c, int q, int t) {
-    unsigned long long key = ((unsigned long long)c.round << 32) | (0xffffffffu - hash32((uint32_t)q));
+    const unsigned long long key = vote_key(c, q);
     if (c.vote[t] != key) return;
-    split_winner(c, q, t, key);
+    const int code = split_rows(c, q, t, c.pedge[q], key);
+    if (code >= 0) c.winners[append_slot(&c.cnt->cur_win, c.base_win)] = make_int2(q * 8 + code, t);
 }
 GCDT_HD void body_split(const Ctx& c, int k) {
     const int q = c.act[k];
@@ -715,9 +746,10 @@ GCDT_HD void resolve_split_edge(const Ctx& c, int ch, int s) {
     }
 }
 
-// Resolve outer adjacency of the children of one inserted point and queue
-// them for the flip phase (c.sr = first sub-round of this round).
-GCDT_HD void body_fix_f(const Ctx& c, int2 w) {
+// Resolve outer adjacency of the children of one inserted point (w: the
+// winner entry) and give the flip-queue entries of the children, qe[0..n-1];
+// returns n (3, or 4 on an edge).
+GCDT_HD int fix_winner(const Ctx& c, int2 w, int4& qe) {
     int q = w.x >> 3, t = w.y;
     int T1 = 2 + 2 * q, T2 = 3 + 2 * q;
     int code = w.x & 7;
@@ -729,41 +761,62 @@ GCDT_HD void body_fix_f(const Ctx& c, int2 w) {
         resolve_split_edge(c, t, 0);
         resolve_split_edge(c, T1, 1);
         resolve_split_edge(c, T2, 2);
-        int* qn = c.queue_next + append_slots(&c.cnt->cur_q, c.base_q, 3);
-        qn[0] = qentry(t, 1); qn[1] = qentry(T1, 2); qn[2] = qentry(T2, 4);
-    } else {
-        int e = code;
-        int e1 = nx3(e), e_2 = nx3(e1);
-        int en = comp(tri_a(c, T1), e);     // A2 slot e = enc(B1, e2)
-        int n = en >> 2, e2 = en & 3;
-        int f1 = nx3(e2), f2 = nx3(f1);
-        resolve_split_edge(c, t, e1);
-        resolve_split_edge(c, T1, e_2);
-        resolve_split_edge(c, n, f1);
-        resolve_split_edge(c, T2, f2);
-        // outer edge and the half of the split edge
-        int* qn = c.queue_next + append_slots(&c.cnt->cur_q, c.base_q, 4);
-        qn[0] = qentry(t, (1 << e1) | (1 << e)); qn[1] = qentry(T1, (1 << e_2) | (1 << e));
-        qn[2] = qentry(n, (1 << f1) | (1 << e2)); qn[3] = qentry(T2, (1 << f2) | (1 << e2));
+        qe = make_int4(qentry(t, 1), qentry(T1, 2), qentry(T2, 4), 0);
+        return 3;
     }
+    int e = code;
+    int e1 = nx3(e), e_2 = nx3(e1);
+    int en = comp(tri_a(c, T1), e);     // A2 slot e = enc(B1, e2)
+    int n = en >> 2, e2 = en & 3;
+    int f1 = nx3(e2), f2 = nx3(f1);
+    resolve_split_edge(c, t, e1);
+    resolve_split_edge(c, T1, e_2);
+    resolve_split_edge(c, n, f1);
+    resolve_split_edge(c, T2, f2);
+    // outer edge and the half of the split edge
+    qe = make_int4(qentry(t, (1 << e1) | (1 << e)), qentry(T1, (1 << e_2) | (1 << e)),
+                   qentry(n, (1 << f1) | (1 << e2)), qentry(T2, (1 << f2) | (1 << e2)));
+    return 4;
+}
+// The same, the entries queued for the flip phase.
+GCDT_HD void body_fix_f(const Ctx& c, int2 w) {
+    int4 qe;
+    const int n = fix_winner(c, w, qe);
+    int* qn = c.queue_next + append_slots(&c.cnt->cur_q, c.base_q, n);
+    qn[0] = qe.x; qn[1] = qe.y; qn[2] = qe.z;
+    if (n == 4) qn[3] = qe.w;
 }
 GCDT_HD void body_fix(const Ctx& c, int k) { body_fix_f(c, c.winners[k]); }
 
 // ---------------------------------------------------------------- flips
 
-// Queue entry t: find the first edge of t that is not locally Delaunay
-// (perturbed incircle > 0, not a constraint) and claim both triangles.
-// The claim priority hash32(4t+i) is unique (hash32 is a bijection); the
-// smallest wins both triangles (atomicMax of its complement), so conflicts
-// resolve like a random-priority independent set, whatever the schedule.
-GCDT_HD void body_flip_check(const Ctx& c, int k) {
-    int qe = c.queue[k];
+GCDT_HD unsigned long long claim_key(const Ctx& c, int key) {
+    return ((unsigned long long)c.sr << 32) | (0xffffffffu - hash32((uint32_t)key));
+}
+
+// The first of the edges `live` of triangle (a, b, cc), in slot order, that
+// is not locally Delaunay (p0, p1, p2: the points opposite them), or -1.  One
+// test per turn, of whichever edge is each lane's next: a warp's entries
+// have different masks (a split's have one edge each, in any slot), and a
+// branch per slot would make every lane wait for three tests.
+GCDT_HD int first_bad_edge(int live, int2 a, int2 b, int2 cc, int2 p0, int2 p1, int2 p2) {
+    while (live) {
+        const int i = (live & 1) ? 0 : ((live & 2) ? 1 : 2);
+        if (incircle_sos(a, b, cc, i == 0 ? p0 : (i == 1 ? p1 : p2)) > 0) return i;
+        live &= live - 1;
+    }
+    return -1;
+}
+
+// The first edge of queue entry qe's triangle that is not locally Delaunay
+// (perturbed incircle > 0, not a constraint): (4t+i, 4n+j) of its two sides,
+// or (-1, -1).  carried: an entry carried over from the previous round, whose
+// triangle may have been split since (then the split's own queue entries
+// test every old edge of it).
+GCDT_HD int2 flip_candidate(const Ctx& c, int qe, bool carried) {
     int t = qtri(qe), mask = qe & 7;
     int4 tv = tri_v(c, t), ta = tri_a(c, t);
-    // a carried entry (first sub-round of a round, before its flips) whose
-    // triangle was split this round: the split's own queue entries test
-    // every old edge of it
-    if (k < c.carry_n && ta.w == (int)c.round) { c.cand[k] = make_int2(-1, -1); return; }
+    if (carried && ta.w == (int)c.round) return make_int2(-1, -1);
     // the edges to test: in the mask, with a neighbour, not constraints
     int live = mask & ~tv.w & ((ta.x >= 0) | ((ta.y >= 0) << 1) | ((ta.z >= 0) << 2));
     // issue every test's loads before the first test, so the neighbour rows
@@ -774,19 +827,23 @@ GCDT_HD void body_flip_check(const Ctx& c, int k) {
     if (live & 4) d2 = comp(tri_v(c, ta.z >> 2), ta.z & 3);
     int2 a = c.P[tv.x], b = c.P[tv.y], cc = c.P[tv.z];
     int2 p0 = c.P[d0], p1 = c.P[d1], p2 = c.P[d2];
-    // first edge in slot order that is not locally Delaunay
-    int i = -1;
-    if ((live & 1) && incircle_sos(a, b, cc, p0) > 0) i = 0;
-    else if ((live & 2) && incircle_sos(a, b, cc, p1) > 0) i = 1;
-    else if ((live & 4) && incircle_sos(a, b, cc, p2) > 0) i = 2;
-    if (i < 0) { c.cand[k] = make_int2(-1, -1); return; }
-    int en = comp(ta, i);
-    int n = en >> 2;
-    int key = enc(t, i);
-    unsigned long long ck = ((unsigned long long)c.sr << 32) | (0xffffffffu - hash32((uint32_t)key));
-    at_max64(&c.claim[t], ck);
-    at_max64(&c.claim[n], ck);
-    c.cand[k] = make_int2(key, en);
+    const int i = first_bad_edge(live, a, b, cc, p0, p1, p2);
+    return i < 0 ? make_int2(-1, -1) : make_int2(enc(t, i), comp(ta, i));
+}
+
+// Queue entry k: claim both triangles of its candidate edge.  The claim
+// priority hash32(4t+i) is unique (hash32 is a bijection); the smallest wins
+// both triangles (atomicMax of its complement), so conflicts resolve like a
+// random-priority independent set, whatever the schedule.
+GCDT_HD void claim_pair(const Ctx& c, int2 cd) {
+    const unsigned long long ck = claim_key(c, cd.x);
+    at_max64(&c.claim[cd.x >> 2], ck);
+    at_max64(&c.claim[cd.y >> 2], ck);
+}
+GCDT_HD void body_flip_check(const Ctx& c, int k) {
+    const int2 cd = flip_candidate(c, c.queue[k], k < c.carry_n);
+    if (cd.x >= 0) claim_pair(c, cd);
+    c.cand[k] = cd;
 }
 
 // Two queue entries per thread (k1 < 0: only k0), each stage's loads issued
@@ -834,10 +891,7 @@ GCDT_HD void flip_check_multi_f(const Ctx& c, const int (&ks)[W], const int2 (&f
     for (int u = 0; u < W; ++u) {
         if (ks[u] < 0) continue;
         if (!on[u]) { c.cand[ks[u]] = make_int2(-1, -1); continue; }   // dropped carried entry
-        int i = -1;
-        if ((live[u] & 1) && incircle_sos(a[u], b[u], cc[u], p[u][0]) > 0) i = 0;
-        else if ((live[u] & 2) && incircle_sos(a[u], b[u], cc[u], p[u][1]) > 0) i = 1;
-        else if ((live[u] & 4) && incircle_sos(a[u], b[u], cc[u], p[u][2]) > 0) i = 2;
+        const int i = first_bad_edge(live[u], a[u], b[u], cc[u], p[u][0], p[u][1], p[u][2]);
         if (i < 0) { c.cand[ks[u]] = make_int2(-1, -1); continue; }
         int en = comp(ta[u], i);
         int n = en >> 2;
@@ -880,19 +934,26 @@ GCDT_HD void body_flip_check_pair(const Ctx& c, int k0, int k1) {
 // every triangle enters the next queue at most once without any
 // de-duplication.
 // The flip of claimed candidate (t slot i, n slot j) given both rows, by
-// value (the rows are overwritten here): writes the two new triangles and
-// their flip maps.
-GCDT_HD void do_flip(const Ctx& c, int t, int i, int n, int j,
-                     const int4 tv, const int4 ta, const int4 nv, const int4 na) {
+// value (the rows are overwritten here): writes the two new triangles, whose
+// outer slots still name the old neighbours, and returns them.
+struct FlipRows { int4 tv, ta, nv, na; };
+GCDT_HD FlipRows do_flip(const Ctx& c, int t, int i, int n, int j,
+                         const int4 tv, const int4 ta, const int4 nv, const int4 na) {
     int i1 = nx3(i), i2 = nx3(i1), j1 = nx3(j), j2 = nx3(j1);
     int A = comp(tv, i), B = comp(tv, i1), C = comp(tv, i2), D = comp(nv, j);
     int ft = tv.w, fn = nv.w;
     // t keeps side 0 of the flip, n side 1; both carry the sub-round
     const int stamp = (int)c.sr << 4;
-    tri_v(c, t) = make_int4(A, B, D, ((fn >> j1) & 1) | (((ft >> i2) & 1) << 2) | stamp);
-    tri_a(c, t) = make_int4(comp(na, j1), enc(n, 2), comp(ta, i2), (int)c.round);
-    tri_v(c, n) = make_int4(A, D, C, ((fn >> j2) & 1) | (((ft >> i1) & 1) << 1) | 8 | stamp);
-    tri_a(c, n) = make_int4(comp(na, j2), comp(ta, i1), enc(t, 1), (int)c.round);
+    FlipRows r;
+    r.tv = make_int4(A, B, D, ((fn >> j1) & 1) | (((ft >> i2) & 1) << 2) | stamp);
+    r.ta = make_int4(comp(na, j1), enc(n, 2), comp(ta, i2), (int)c.round);
+    r.nv = make_int4(A, D, C, ((fn >> j2) & 1) | (((ft >> i1) & 1) << 1) | 8 | stamp);
+    r.na = make_int4(comp(na, j2), comp(ta, i1), enc(t, 1), (int)c.round);
+    tri_v(c, t) = r.tv;
+    tri_a(c, t) = r.ta;
+    tri_v(c, n) = r.nv;
+    tri_a(c, n) = r.na;
+    return r;
 }
 
 // The edge in slot s of flipped triangle tt (vertex row tv) had the old
@@ -940,29 +1001,37 @@ GCDT_HD void body_flip_do(const Ctx& c, int k) {
     qn[1] = qentry(n, 3);    // (A,D,C): DC and CA
 }
 
-// Two candidates per thread (k1 < 0: only k0): the candidate and claim
-// loads of both are in flight together; the winners (a minority) then
-// flip one at a time, so only one pair of rows is live at once.
-GCDT_HD void body_flip_do_pair_f(const Ctx& c, const int (&ks)[2], const int2 (&first)[2]) {
-    int2 cd[2];
+// W candidates per thread (k < 0: none): the candidate and claim loads of
+// all are in flight together; the winners (a minority) then flip one at a
+// time, so only one pair of rows is live at once.
+template <int W>
+GCDT_HD void flip_do_multi_f(const Ctx& c, const int (&ks)[W], const int2 (&first)[W]) {
+    int2 cd[W];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) cd[u] = ks[u] >= 0 ? first[u] : make_int2(-1, -1);
-    bool win[2];
+    for (int u = 0; u < W; ++u) cd[u] = ks[u] >= 0 ? first[u] : make_int2(-1, -1);
+    unsigned win = 0;
+    int nw = 0;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        unsigned long long ck = ((unsigned long long)c.sr << 32) | (0xffffffffu - hash32((uint32_t)cd[u].x));
+    for (int u = 0; u < W; ++u) {
+        const unsigned long long ck = claim_key(c, cd[u].x);
         unsigned long long c0 = cd[u].x >= 0 ? c.claim[cd[u].x >> 2] : 0ull;
         unsigned long long c1 = cd[u].x >= 0 ? c.claim[cd[u].y >> 2] : 0ull;
-        win[u] = cd[u].x >= 0 && c0 == ck && c1 == ck;
+        const bool w = cd[u].x >= 0 && c0 == ck && c1 == ck;
+        win |= (unsigned)w << u;
+        nw += (int)w;
     }
-    const int nw = (int)win[0] + (int)win[1];
     if (nw == 0) return;
     int f = append_slots(&c.cnt->cur_flip, c.base_flip, nw);
-#pragma unroll 1
-    for (int u = 0; u < 2; ++u) {
-        if (!win[u]) continue;
-        int t = cd[u].x >> 2, n = cd[u].y >> 2;
-        do_flip(c, t, cd[u].x & 3, n, cd[u].y & 3, tri_v(c, t), tri_a(c, t), tri_v(c, n), tri_a(c, n));
+    // winner by winner, picked by selects (an index computed at run time
+    // would put the candidates in local memory)
+    while (win) {
+        int2 x = cd[0];
+#pragma unroll
+        for (int u = 1; u < W; ++u)
+            if (!(win & ((1u << u) - 1u))) x = cd[u];
+        win &= win - 1;
+        int t = x.x >> 2, n = x.y >> 2;
+        do_flip(c, t, x.x & 3, n, x.y & 3, tri_v(c, t), tri_a(c, t), tri_v(c, n), tri_a(c, n));
         int* qn = c.queue_next + 2 * f++;
         qn[0] = qentry(t, 5);
         qn[1] = qentry(n, 3);
@@ -972,7 +1041,7 @@ GCDT_HD void body_flip_do_pair_f(const Ctx& c, const int (&ks)[2], const int2 (&
 GCDT_HD void body_flip_do_pair(const Ctx& c, int k0, int k1) {
     const int ks[2] = {k0, k1};
     const int2 f[2] = {flip_first(c, FP_DO, k0), flip_first(c, FP_DO, k1)};
-    body_flip_do_pair_f(c, ks, f);
+    flip_do_multi_f<2>(c, ks, f);
 }
 
 GCDT_HD void resolve_flip_edge(const Ctx& c, int tt, int s) {
@@ -1014,14 +1083,15 @@ GCDT_HD void resolve_flip_loaded(const Ctx& c, int tt, const int4& tv, int s, in
     else ((int*)&tri_a(c, old >> 2))[old & 3] = enc(tt, s);
 }
 
-// Two items per thread (k1 < 0: only k0), as body_flip_fix on each, with
-// every stage's loads issued for both items first.
-GCDT_HD void body_flip_fix_pair_f(const Ctx& c, const int (&ks)[2], const int2 (&f)[2]) {
+// W items per thread (k < 0: none), as body_flip_fix on each, with every
+// stage's loads issued for all of them first.
+template <int W>
+GCDT_HD void flip_fix_multi_f(const Ctx& c, const int (&ks)[W], const int2 (&f)[W]) {
     const int4 none = make_int4(-1, -1, -1, -1);
-    int kind[2], t[2], n[2];    // kind 0: nothing, 1: flipped pair, 2: candidate of the queue
-    int2 cd[2];
+    int kind[W], t[W], n[W];    // kind 0: nothing, 1: flipped pair, 2: candidate of the queue
+    int2 cd[W];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < W; ++u) {
         kind[u] = ks[u] < 0 ? 0 : (ks[u] >= c.list_n ? 2 : 1);
         cd[u] = kind[u] == 2 ? f[u] : make_int2(-1, -1);
         t[u] = kind[u] == 1 ? qtri(f[u].x) : 0;
@@ -1029,10 +1099,10 @@ GCDT_HD void body_flip_fix_pair_f(const Ctx& c, const int (&ks)[2], const int2 (
     }
     // both triangles of a flipped pair at once (the pair's two queue entries
     // name them), so their old neighbours are one load further on
-    int4 tv[2], ta[2], nv[2], na[2];
-    int flw[2];
+    int4 tv[W], ta[W], nv[W], na[W];
+    int flw[W];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < W; ++u) {
         tv[u] = kind[u] == 1 ? tri_v(c, t[u]) : none;
         ta[u] = kind[u] == 1 ? tri_a(c, t[u]) : none;
         nv[u] = kind[u] == 1 ? tri_v(c, n[u]) : none;
@@ -1040,32 +1110,35 @@ GCDT_HD void body_flip_fix_pair_f(const Ctx& c, const int (&ks)[2], const int2 (
         flw[u] = (kind[u] == 2 && cd[u].x >= 0) ? tri_v(c, cd[u].x >> 2).w : 0;
     }
     // re-queue the candidates that did not flip and whose triangle nobody flipped
-    int rq[2];
+    int rq[W];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) rq[u] = (kind[u] == 2 && cd[u].x >= 0 && flip_stamp(flw[u]) != (int)c.sr) ? 1 : 0;
-    if (rq[0] | rq[1]) {
-        int at = 2 * c.list_n + append_slots(&c.cnt->cur_q, c.base_q, rq[0] + rq[1]);
+    for (int u = 0; u < W; ++u) rq[u] = (kind[u] == 2 && cd[u].x >= 0 && flip_stamp(flw[u]) != (int)c.sr) ? 1 : 0;
+    int nrq = 0;
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+    for (int u = 0; u < W; ++u) nrq += rq[u];
+    if (nrq) {
+        int at = 2 * c.list_n + append_slots(&c.cnt->cur_q, c.base_q, nrq);
+#pragma unroll
+        for (int u = 0; u < W; ++u)
             if (rq[u]) c.queue_next[at++] = c.queue[ks[u] - c.list_n];
     }
     // flipped pairs: t's outer edges 0, 2 and n's outer edges 0, 1; each old
     // neighbour's row (one sector, which the fix writes when that neighbour
     // did not flip) tells whether it flipped and where the edge went
-    int4 m0[2], m2[2];
-    int2 p0[2], p2[2];
+    int4 m0[W], m2[W];
+    int2 p0[W], p2[W];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < W; ++u) {
         const bool l0 = kind[u] == 1 && ta[u].x >= 0, l2 = kind[u] == 1 && ta[u].z >= 0;
         m0[u] = l0 ? tri_v(c, ta[u].x >> 2) : none;
         p0[u] = l0 ? partner_slots(c, ta[u].x >> 2) : make_int2(-1, -1);
         m2[u] = l2 ? tri_v(c, ta[u].z >> 2) : none;
         p2[u] = l2 ? partner_slots(c, ta[u].z >> 2) : make_int2(-1, -1);
     }
-    int4 g0[2], g1[2];
-    int2 q0[2], q1[2];
+    int4 g0[W], g1[W];
+    int2 q0[W], q1[W];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < W; ++u) {
         const bool l0 = kind[u] == 1 && na[u].x >= 0, l1 = kind[u] == 1 && na[u].y >= 0;
         g0[u] = l0 ? tri_v(c, na[u].x >> 2) : none;
         q0[u] = l0 ? partner_slots(c, na[u].x >> 2) : make_int2(-1, -1);
@@ -1073,7 +1146,7 @@ GCDT_HD void body_flip_fix_pair_f(const Ctx& c, const int (&ks)[2], const int2 (
         q1[u] = l1 ? partner_slots(c, na[u].y >> 2) : make_int2(-1, -1);
     }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < W; ++u) {
         if (kind[u] != 1) continue;
         resolve_flip_loaded(c, t[u], tv[u], 0, ta[u].x, m0[u], p0[u]);
         resolve_flip_loaded(c, t[u], tv[u], 2, ta[u].z, m2[u], p2[u]);
@@ -1085,7 +1158,7 @@ GCDT_HD void body_flip_fix_pair_f(const Ctx& c, const int (&ks)[2], const int2 (
 GCDT_HD void body_flip_fix_pair(const Ctx& c, int k0, int k1) {
     const int ks[2] = {k0, k1};
     const int2 f[2] = {flip_first(c, FP_FIX, k0), flip_first(c, FP_FIX, k1)};
-    body_flip_fix_pair_f(c, ks, f);
+    flip_fix_multi_f<2>(c, ks, f);
 }
 
 // ---------------------------------------------------------------- constraints

@@ -188,6 +188,13 @@ GCDT_HD void run_phase(EX& ex, Ctx& c, Driver& D, int k, long long count) {
     D.nphase++;
 }
 
+// An executor with kFastItems runs short lists by whole sub-rounds and
+// rounds (fast_flips, fast_round), with the same result as the phases.
+template <class EX, class = void>
+struct FastItems { static constexpr int value = 0; };
+template <class EX>
+struct FastItems<EX, decltype((void)EX::kFastItems)> { static constexpr int value = EX::kFastItems; };
+
 // Flip sub-rounds on the queue `D.qa` (nq entries, stamped D.sr) until it
 // has at most `stop` entries after at least one sub-round, or -- for the
 // single-block tail -- until it grows past max_nq.  The first sub-round
@@ -202,6 +209,15 @@ GCDT_HD int flip_loop(EX& ex, Ctx& c, Driver& D, long long& nq, long long max_nq
             int rc = ex.narrow_flips(c, D, nq);
             if (rc || D.errs) return rc ? rc : D.errs;
             continue;
+        }
+        if constexpr (FastItems<EX>::value > 0) {
+            if (nq <= FastItems<EX>::value && nq <= max_nq && stop == 0) {
+                long long left = budget - guard + 1;
+                const int rc = ex.fast_flips(c, D, nq, left);
+                if (rc) return rc;
+                guard = budget - left;
+                continue;
+            }
         }
         c.queue = D.qa; c.queue_next = D.qb; c.sr = D.sr;
         c.base_q = D.e_q;
@@ -247,6 +263,21 @@ GCDT_HD int insert_rounds(EX& ex, Ctx& c, Driver& D, long long nact) {
         }
         if (++D.round > budget_rounds(c)) return ST_ITER_LIMIT;
         c.round = D.round;
+        if constexpr (FastItems<EX>::value > 0) {
+            if (nact <= FastItems<EX>::value) {
+                long long nq = 0;
+                const int alive = ex.fast_round(c, D, nact, nq);
+                if (D.errs) return D.errs;
+                if (alive == 0) break;
+                D.sr++;
+                D.rounds++;
+                const int rc = flip_until_delaunay(ex, c, D, nq);
+                if (rc) return rc;
+                // the phases find an empty list in a round of its own
+                if (nact == 0 && ++D.round > budget_rounds(c)) return ST_ITER_LIMIT;
+                continue;
+            }
+        }
         c.act = D.actA; c.act_next = D.actB;
         c.base_act = D.e_act;
         run_phase(ex, c, D, K_RELOC_VOTE, nact);

@@ -1,0 +1,99 @@
+"""The executors that run a solve on the GPU -- the whole grid, a cluster, one
+block, and the whole-round commands of short lists -- follow one history: at
+the sizes where a solve passes from one to another its output has the bytes
+of the sequential host run of the same bodies (tests/host_emulation.cu)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import gcdt_b200 as g
+from tests.test_host_emulation import build_host_emulation
+
+pytestmark = pytest.mark.gpu
+
+
+def _host(xy, cons, tuning=None):
+    L = ctypes.CDLL(build_host_emulation())
+    vp, i32 = ctypes.c_void_p, ctypes.c_int
+    L.host_triangulate.argtypes = [vp, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32]
+    L.host_set_tuning.argtypes = [i32] * 7
+    T = 2 * len(xy) + 2
+    out = (np.zeros((T, 3), np.int32), np.zeros((T, 3), np.int32), np.zeros(T, np.uint8))
+    st = np.zeros(8, np.int64)
+    p = lambda a: ctypes.c_void_p(a.ctypes.data)
+    L.host_set_tuning(*(tuning or (0,) * 7))
+    rc = L.host_triangulate(p(xy), len(xy), p(cons), len(cons), *map(p, out), p(st), 0, 2, 0)
+    L.host_set_tuning(*(0,) * 7)
+    assert rc == 0
+    return out
+
+
+def _instance(n, seed):
+    if n < 64:
+        rng = np.random.default_rng(seed)
+        xy = rng.integers(1, 1 << 24, size=(n, 2)).astype(np.int32)
+        return xy, np.zeros((0, 2), np.int32)
+    xy, cons = g.generate(g.GEN_BATCH_INSTANCE, seed, n)
+    return np.ascontiguousarray(xy), np.ascontiguousarray(cons)
+
+
+def _equal(got, want):
+    return all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+# one block's list capacity is 512, the tails' default threshold 1,024; a
+# cluster solves up to 15,000 points
+@pytest.mark.parametrize("n", [1, 2, 3, 64, 480, 512, 513, 1024, 1025, 4000, 14800, 14999, 15000, 15001, 40000])
+def test_single_solve_has_the_host_bytes(n):
+    xy, cons = _instance(n, 3 * n)
+    if n > 14000:       # exact point counts on both sides of the cluster's limit
+        xy, cons = xy[:n], np.zeros((0, 2), np.int32)
+    tri = g.Triangulator(len(xy), max(len(cons), 1))
+    got = tri.triangulate_host(xy, cons)
+    tri.close()
+    assert _equal(got, _host(xy, cons))
+
+
+@pytest.mark.parametrize("narrow", [0, 300, 4096, 65536])
+def test_single_block_tails_of_every_length(narrow):
+    """Tails that start above the block's list capacities (long lists in
+    device memory, short ones in shared, and the passage between them)."""
+    xy, cons = _instance(20000, 77)
+    t = (3, 512, 8, 1, 1 << 22, narrow, narrow)
+    tri = g.Triangulator(len(xy), len(cons))
+    tri.set_tuning(narrow_queue=narrow, narrow_active=narrow)
+    got = tri.triangulate_host(xy, cons)
+    tri.close()
+    assert _equal(got, _host(xy, cons, t))
+
+
+@pytest.mark.parametrize("threads,stride", [(128, 16), (256, 64), (512, 16)])
+def test_batch_instances_have_the_host_bytes(threads, stride):
+    """Clusters of eight, four and two blocks and single blocks in one batch
+    (an instance's share of 200 decides), against the host run of the batch's
+    schedule: two levels, nothing carried."""
+    inst = [_instance(n, 900 + n) for n in (30000, 15000, 8000, 2600, 1999, 700, 481, 64, 3, 1)]
+    po, so = g.BatchTriangulator.offsets(inst)
+    bt = g.BatchTriangulator(len(inst), int(po[-1]), int(so[-1]))
+    bt.set_config(threads, stride)
+    res = bt.triangulate(inst)
+    bt.close()
+    for (xy, cons), r in zip(inst, res):
+        assert not isinstance(r, Exception), r
+        assert _equal(r, _host(xy, cons, (2, stride, 1, 1, 0, 1024, 1024))), len(xy)
+
+
+def test_batch_of_mixed_cluster_sizes():
+    """Enough instances that the share of the batch separates the cluster
+    sizes: each instance again has the host run's bytes."""
+    sizes = [12000] * 2 + [6000] * 6 + [3000] * 30 + [2100] * 60 + [1500] * 300 + [200] * 100
+    inst = [_instance(n, 5000 + i) for i, n in enumerate(sizes)]
+    po, so = g.BatchTriangulator.offsets(inst)
+    bt = g.BatchTriangulator(len(inst), int(po[-1]), int(so[-1]))
+    bt.set_config(512, 16)
+    res = bt.triangulate(inst)
+    bt.close()
+    for i in (0, 1, 2, 7, 8, 37, 38, 97, 98, 397, 398, 497):
+        xy, cons = inst[i]
+        assert _equal(res[i], _host(xy, cons, (2, 16, 1, 1, 0, 1024, 1024))), (i, len(xy))
