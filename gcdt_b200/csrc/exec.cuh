@@ -262,8 +262,8 @@ struct BlockExecT {
 // the time of a solve of up to about 100,000 points and the tails of every
 // level; their phases are a few hundred dependent instructions on a few
 // warps, so publishing each phase, its lists in memory and generic
-// addressing cost more than its work (a flip sub-round of the tails 5.6 -> 2.2 us: check 1.1, flip 0.45, fix
-// 0.65; a round's insertion 9 -> 4.8 us).
+// addressing cost more than its work (a flip sub-round of the tails 5.6 ->
+// 2.2 us: check 1.1, flip 0.45, fix 0.65; a round's insertion 9 -> 4.8 us).
 
 constexpr int kBarFast = 3;
 template <int CAP>
@@ -600,11 +600,12 @@ struct TeamExec {
     Counters* cnt;
     unsigned rank, size;                     // of the block in its team, of the team
     SH* sh;
-    unsigned spin_limit = 1u << 24;          // polls before a grid barrier wait gives up
+    unsigned spin_limit = 1u << 25;          // polls before a grid barrier wait gives up
     bool prof = false;                       // record the phase profile and balance (a launch constant)
     // Snapshot of the head of Counters (status, error words, list cursors),
     // word k in lane k, read right after each barrier.
     unsigned long long snap = 0;
+    unsigned parity = 0;                     // of the grid barriers passed, in the top bit
 
     __device__ int narrow_flips(Ctx& c, Driver& D, long long& nq);
     __device__ int narrow_rounds(Ctx& c, Driver& D, long long nact);
@@ -617,16 +618,18 @@ struct TeamExec {
     // Grid barrier on one counter whose top bit flips once per barrier:
     // block 0 adds 2^31 - (blocks - 1), every other block adds 1, so the
     // count's low 31 bits are back at 0 and its top bit has flipped once
-    // every block has arrived, and a block waits for the top bit to differ
-    // from the value its own add saw.  One atomic per block and no reset
-    // (2.9 -> 2.35 us per barrier against a counter reset by the last
-    // arrival plus a generation word).  The counter starts each launch at
-    // 0 (the solve clears its counters).  Every wait is bounded: after
-    // spin_limit polls (2^24, about a second, in a solve) the block records
-    // ST_BARRIER and stops waiting, and once that bit is set no block waits
-    // or works any more, so the kernel always ends.  The driver warp alone
-    // takes part: the block's workers have reported to it (kBarDone) and
-    // wait for the next phase.
+    // every block has arrived, and a block waits for the top bit to reach
+    // the barrier's parity, which its driver counts along.  One atomic per
+    // block, whose result nobody waits for, and no reset.  The counter starts
+    // each launch at 0 (the solve clears its counters).  Every wait is
+    // bounded: after spin_limit polls (2^25, about ten seconds, in a solve)
+    // the block records ST_BARRIER and stops waiting, and once that bit is
+    // set no block waits or works any more, so the kernel always ends.  A
+    // poll is one L2 round trip and nothing else: sleeping 64 ns between
+    // polls, reading the status word with each, and waiting for the add's
+    // result before the first cost 2.70 against 1.87 us per barrier.  The
+    // driver warp alone takes part: the block's workers have reported to it
+    // (kBarDone) and wait for the next phase.
     // In a cluster the hardware's barrier, which the workers take part in as
     // well (they go to it from their items, or are sent by kTeamSync).
     __device__ void barrier() {
@@ -645,24 +648,20 @@ struct TeamExec {
         take_snapshot();
     }
     __device__ void grid_barrier() {
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) {
+        const bool off = (word(&cnt->status) & ST_BARRIER) != 0;
+        parity ^= 0x80000000u;
+        if ((threadIdx.x & 31) == 0 && !off) {
+            const unsigned add = rank == 0 ? 0x80000000u - (size - 1) : 1u;
+            asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u32 [%0], %1;"
+                         :: "l"(__cvta_generic_to_global(&cnt->bar_count)), "r"(add) : "memory");
             volatile unsigned* vcount = &cnt->bar_count;
             volatile int* vst = &cnt->status;
-            if (!(*vst & ST_BARRIER)) {
-                const unsigned add = rank == 0 ? 0x80000000u - (size - 1) : 1u;
-                __threadfence();
-                const unsigned old = atomicAdd(&cnt->bar_count, add);
-                // the arrival that completes the count flips the top bit itself
-                const bool last = (((old + add) ^ old) & 0x80000000u) != 0;
-                unsigned spins = 0;
-                while (!last && ((old ^ *vcount) & 0x80000000u) == 0) {
-                    if (++spins > spin_limit) { atomicOr(&cnt->status, ST_BARRIER); break; }
-                    if (*vst & ST_BARRIER) break;
-                    __nanosleep(64);
-                }
+            unsigned spins = 0;
+            while (((*vcount ^ parity) & 0x80000000u) != 0) {
+                if (++spins > spin_limit) { atomicOr(&cnt->status, ST_BARRIER); break; }
+                if ((spins & 63u) == 0 && (*vst & ST_BARRIER)) break;
             }
-            __threadfence();
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
         }
         // the snapshot words read by twelve lanes at once, after lane 0 has
         // seen the barrier open (3.20 -> 2.90 us per barrier against one
