@@ -100,14 +100,29 @@ __device__ int solve_instance(EX& ex, const Ctx& c) {
     return st ? st : run_stages(ex, c);
 }
 
+// A batch's kernels (clusters of eight, of four, of two, single blocks) are
+// launched in a row with programmatic stream serialization: each may start
+// as soon as all blocks of the one before it have, so that the order is the
+// largest instance first and no kernel waits for another's last instance.
+// Nothing in them depends on an earlier one; block 0 waits for it at its end,
+// so that what follows on the stream waits for all of them.
+__device__ __forceinline__ void start_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous_kernel() {
+    if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // BS threads, the last warp the driver.  What bounds an instance is latency
 // (its mesh sits in L2), so two blocks of 512 threads share an SM at 64
 // registers: 4,096 instances 86.8 -> 67.1 ms against one block at 128, and
 // three at 40 registers spill (67.6).
 template <int BS>
 __global__ void __launch_bounds__(BS, 1024 / BS) gcdt_batch_solve(BatchArgs a, int first) {
+    start_next_kernel();
     const int inst = a.order[first + blockIdx.x];
-    if (a.desc[inst].status) return;             // rejected by the key pass
+    if (a.desc[inst].status) {                   // rejected by the key pass
+        wait_previous_kernel();
+        return;
+    }
     __shared__ BlockShared<BS - 32> sh;
     if (threadIdx.x == 0) {
         sh.ctx = instance_ctx(a, inst);
@@ -131,6 +146,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) gcdt_batch_solve(BatchArgs a, i
     if (threadIdx.x == BS - 32) a.desc[inst].status = st;
     publish(sh, kExit, c, 0, true);
     block_sync(kBarWork);
+    wait_previous_kernel();
 }
 
 // A cluster phase's items read the context from shared memory; its lists are
@@ -162,9 +178,13 @@ struct SharedView {
 // that either fills the room the other leaves.
 constexpr int kClusterThreads = 512;
 __global__ void __launch_bounds__(kClusterThreads, 2) gcdt_batch_cluster(BatchArgs a, int first) {
+    start_next_kernel();
     const unsigned rank = cluster_rank(), size = cluster_size();
     const int inst = a.order[first + blockIdx.x / size];
-    if (a.desc[inst].status) return;             // rejected by the key pass
+    if (a.desc[inst].status) {                   // rejected by the key pass
+        wait_previous_kernel();
+        return;
+    }
     constexpr int kWork = kClusterThreads - 32;
     using SH = BlockShared<kWork>;
     __shared__ SH sh;
@@ -187,15 +207,12 @@ __global__ void __launch_bounds__(kClusterThreads, 2) gcdt_batch_cluster(BatchAr
     if (rank == 0 && threadIdx.x == kWork) a.desc[inst].status = st;
     publish(sh, kExit, c, 0, false);
     block_sync(kBarWork);
+    wait_previous_kernel();
 }
 
 }  // namespace gcdt
 
 using namespace gcdt;
-
-namespace {
-constexpr int kClusterSizes = 3;     // of 8, 4 and 2 blocks
-}
 
 struct gcdt_batch {
     int device = 0;
@@ -213,10 +230,6 @@ struct gcdt_batch {
     int* h_order = nullptr;          // pinned
     gcdt_batch_config cfg{256, 64};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // the clusters' launches run beside the single blocks': one stream and
-    // event per cluster size
-    cudaStream_t side[kClusterSizes] = {};
-    cudaEvent_t fork = nullptr, join[kClusterSizes] = {};
     double last_ms = 0.0;
 };
 
@@ -350,48 +363,35 @@ gcdt_status gcdt_batch_launch(gcdt_batch* b, int32_t ninst, const int64_t* pt_of
     a.adj = d_adj;
     a.cflags = d_cflags;
     a.stride0 = cfg.sample_stride;
-    // The largest instances, one per cluster, on streams of their own next
-    // to the other instances' blocks; the instances are in order of size.
+    // The instances are in order of size: clusters first, single blocks last,
+    // one launch per cluster size (see start_next_kernel).
     cudaError_t e = cudaSuccess;
-    int at = 0;
-    bool forked = false, joined[kClusterSizes] = {};
-    for (int k = 0; k < kClusterSizes && e == cudaSuccess; ++k) {
-        const int size = 8 >> k;
-        int end = at;
+    for (int size = 8, at = 0; size >= 1 && e == cudaSuccess; size >>= 1) {
+        int end = size == 1 ? ninst : at;
         while (end < ninst && cluster_blocks(b->h_desc[b->h_order[end]].n, total) >= size) ++end;
         if (end == at) continue;
-        if (!forked) e = cudaEventRecord(b->fork, st);
-        forked = true;
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(b->side[k], b->fork, 0);
-        if (e != cudaSuccess) break;
-        joined[k] = true;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = size;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cudaLaunchAttribute attr[2];
         cudaLaunchConfig_t lc{};
         lc.gridDim = dim3((unsigned)(end - at) * size);
-        lc.blockDim = dim3(kClusterThreads);
-        lc.stream = b->side[k];
+        lc.blockDim = dim3(size > 1 ? kClusterThreads : cfg.threads_per_instance);
+        lc.stream = st;
         lc.attrs = attr;
-        lc.numAttrs = 1;
-        e = cudaLaunchKernelEx(&lc, gcdt_batch_cluster, a, at);
-        at = end;
-    }
-    if (e == cudaSuccess && at < ninst) {
-        const int m = ninst - at;
-        switch (cfg.threads_per_instance) {
-        case 128: gcdt_batch_solve<128><<<m, 128, 0, st>>>(a, at); break;
-        case 512: gcdt_batch_solve<512><<<m, 512, 0, st>>>(a, at); break;
-        default: gcdt_batch_solve<256><<<m, 256, 0, st>>>(a, at); break;
+        if (size > 1) {
+            attr[lc.numAttrs].id = cudaLaunchAttributeClusterDimension;
+            attr[lc.numAttrs].val.clusterDim.x = size;
+            attr[lc.numAttrs].val.clusterDim.y = attr[lc.numAttrs].val.clusterDim.z = 1;
+            ++lc.numAttrs;
         }
-        e = cudaGetLastError();
-    }
-    for (int k = 0; k < kClusterSizes; ++k) {
-        if (!joined[k]) continue;
-        cudaError_t j = cudaEventRecord(b->join[k], b->side[k]);
-        if (j == cudaSuccess) j = cudaStreamWaitEvent(st, b->join[k], 0);
-        if (e == cudaSuccess) e = j;
+        if (at > 0) {
+            attr[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[lc.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+            ++lc.numAttrs;
+        }
+        if (size > 1) e = cudaLaunchKernelEx(&lc, gcdt_batch_cluster, a, at);
+        else if (cfg.threads_per_instance == 128) e = cudaLaunchKernelEx(&lc, gcdt_batch_solve<128>, a, at);
+        else if (cfg.threads_per_instance == 512) e = cudaLaunchKernelEx(&lc, gcdt_batch_solve<512>, a, at);
+        else e = cudaLaunchKernelEx(&lc, gcdt_batch_solve<256>, a, at);
+        at = end;
     }
     if (e != cudaSuccess) return GCDT_CUDA_ERROR;
     cudaMemcpyAsync(b->h_desc, b->d_desc, sizeof(BatchDesc) * ninst, cudaMemcpyDeviceToHost, st);
@@ -448,11 +448,7 @@ extern "C" gcdt_status gcdt_batch_create(gcdt_batch** out, int device, int64_t m
               cudaMallocHost(&b->h_desc, sizeof(BatchDesc) * max_instances) == cudaSuccess &&
               cudaMallocHost(&b->h_offs, 4 * (max_instances + 1)) == cudaSuccess &&
               cudaMallocHost(&b->h_order, 4 * max_instances) == cudaSuccess &&
-              cudaEventCreate(&b->ev0) == cudaSuccess && cudaEventCreate(&b->ev1) == cudaSuccess &&
-              cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) == cudaSuccess;
-    for (int k = 0; k < kClusterSizes; ++k)
-        ok = ok && cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) == cudaSuccess &&
-             cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming) == cudaSuccess;
+              cudaEventCreate(&b->ev0) == cudaSuccess && cudaEventCreate(&b->ev1) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         gcdt_batch_destroy(b);
@@ -476,11 +472,6 @@ extern "C" void gcdt_batch_destroy(gcdt_batch* b) {
     if (b->h_order) cudaFreeHost(b->h_order);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
-    if (b->fork) cudaEventDestroy(b->fork);
-    for (int k = 0; k < kClusterSizes; ++k) {
-        if (b->side[k]) cudaStreamDestroy(b->side[k]);
-        if (b->join[k]) cudaEventDestroy(b->join[k]);
-    }
     delete b;
 }
 
