@@ -14,19 +14,91 @@ namespace gcdt {
 
 constexpr int kBlock = 256;
 
-#define GCDT_KERNEL(name, body)                                            \
-    __global__ void __launch_bounds__(kBlock) name(Ctx c, int n) {         \
-        int i = blockIdx.x * kBlock + threadIdx.x;                         \
-        if (i < n) body(c, i);                                             \
+// The set-up before the stages, for problems whose sort takes the whole GPU:
+// clears and keys, (the sort,) points in order with their levels, segments.
+// (The counters are cleared before: the keys report errors in them.)
+__global__ void __launch_bounds__(kBlock) gcdt_keys(Ctx c) {
+    const long long i = (long long)blockIdx.x * kBlock + threadIdx.x, stride = (long long)gridDim.x * kBlock;
+    if (i < c.n) body_keys(c, (int)i);
+    for (long long t = i; t < c.ntri; t += stride) body_clear(c, (int)t);
+}
+__global__ void __launch_bounds__(kBlock) gcdt_points(Ctx c) {
+    const int i = blockIdx.x * kBlock + threadIdx.x;
+    if (i >= c.n + 4) return;
+    body_gather(c, i);
+    if (i < c.n) body_level(c, i);
+    if (i == 0) body_root(c, 0);
+}
+__global__ void __launch_bounds__(kBlock) gcdt_segments(Ctx c) {
+    const int k = blockIdx.x * kBlock + threadIdx.x;
+    if (k >= c.s) return;
+    body_seg_init(c, k);
+    body_seg_level0(c, k);
+}
+
+// The same for problems whose device sort (60 bits: eight passes, and as many
+// launches again) takes longer than comparing all pairs of keys: a point's
+// sorted position is the number of smaller keys.  The set-up of 4,000 points
+// took 140 us in twelve kernels, now 30 in four (10 of them the comparisons);
+// at 16,000 points it is 85 us shorter, at about 30,000 the n^2 comparisons
+// would take what the sort does.  250 points: 60 -> 25 us (in one block with
+// a bitonic sort 30, and 61 at 4,000).
+constexpr int kRankPoints = 16384;
+constexpr int kRankTile = 1024;
+__global__ void __launch_bounds__(kBlock) gcdt_rank_keys(Ctx c) {
+    const int i = blockIdx.x * kBlock + threadIdx.x;
+    if (i < c.n) {
+        c.keys[i] = sort_key60(c.in_xy[i]);
+        c.rank[i] = 0;
+        c.perm[i] = -1;
     }
+    for (int t = i; t < c.ntri; t += gridDim.x * kBlock) body_clear(c, t);
+    for (int k = i; k < (int)(sizeof(Counters) / 8); k += gridDim.x * kBlock)
+        reinterpret_cast<unsigned long long*>(c.cnt)[k] = 0;
+}
+// Block (x, y): points of x against the tile of keys y.
+__global__ void __launch_bounds__(kBlock) gcdt_rank(Ctx c) {
+    __shared__ unsigned long long tile[kRankTile];
+    const int first = blockIdx.y * kRankTile;
+    for (int k = threadIdx.x; k < kRankTile; k += kBlock) tile[k] = first + k < c.n ? c.keys[first + k] : ~0ull;
+    __syncthreads();
+    const int i = blockIdx.x * kBlock + threadIdx.x;
+    if (i >= c.n) return;
+    const unsigned long long key = c.keys[i];
+    int smaller = 0;
+#pragma unroll 16
+    for (int k = 0; k < kRankTile; ++k) smaller += tile[k] < key;
+    if (smaller) atomicAdd(&c.rank[i], smaller);
+}
+__global__ void __launch_bounds__(kBlock) gcdt_rank_points(Ctx c) {
+    const int i = blockIdx.x * kBlock + threadIdx.x;
+    if (i < c.n) {
+        const int2 p = c.in_xy[i];
+        check_range(c, p);
+        const int r = c.rank[i];
+        c.P[r] = p;
+        c.perm[r] = i;
+        body_level(c, r);
+    } else if (i < c.n + 4) {
+        body_gather(c, i);          // a corner
+    }
+    if (i == 0) body_root(c, 0);
+}
+// Equal points have one position between them and leave another empty.
+__global__ void __launch_bounds__(kBlock) gcdt_rank_check(Ctx c) {
+    const int k = blockIdx.x * kBlock + threadIdx.x;
+    if (k < c.n && c.perm[k] < 0) fail(c, ST_BAD_INPUT);
+    if (k >= c.s) return;
+    body_seg_init(c, k);
+    body_seg_level0(c, k);
+}
 
-GCDT_KERNEL(gcdt_keys, body_keys)
-GCDT_KERNEL(gcdt_gather, body_gather)
-GCDT_KERNEL(gcdt_root, body_root)
-GCDT_KERNEL(gcdt_level, body_level)
-GCDT_KERNEL(gcdt_seg_level0, body_seg_level0)
-GCDT_KERNEL(gcdt_seg_init, body_seg_init)
-
+// The whole set-up of a small problem in one block: its launches took longer
+// than their work (eleven launches and a 60-bit device sort of eight passes,
+// 140 us at 4,000 points and 60 at 250; this kernel FILL and FILL).  The sort
+// is a bitonic network over (key, index) pairs in shared memory; its steps
+// of stride up to 32 stay inside a warp's 64 entries and need no block
+// barrier.
 __global__ void gcdt_predicates(const int2* q, int n, int* out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -101,23 +173,29 @@ struct DeviceBackend {
 
     void note(cudaError_t e) { if (e != cudaSuccess && err == cudaSuccess) err = e; }
 
-    void launch(int k, const Ctx& c, long long n) {
-        if (n <= 0 || err != cudaSuccess) return;
-        unsigned grid = (unsigned)((n + kBlock - 1) / kBlock);
-        int nn = (int)n;
-        switch (k) {
-        case K_KEYS: gcdt_keys<<<grid, kBlock, 0, st>>>(c, nn); break;
-        case K_GATHER: gcdt_gather<<<grid, kBlock, 0, st>>>(c, nn); break;
-        case K_ROOT: gcdt_root<<<grid, kBlock, 0, st>>>(c, nn); break;
-        case K_LEVEL: gcdt_level<<<grid, kBlock, 0, st>>>(c, nn); break;
-        case K_SEG_LEVEL0: gcdt_seg_level0<<<grid, kBlock, 0, st>>>(c, nn); break;
-        case K_SEG_INIT: gcdt_seg_init<<<grid, kBlock, 0, st>>>(c, nn); break;
-        default: note(cudaErrorInvalidValue); return;
-        }
+    void launch(void (*kern)(Ctx), dim3 grid, const Ctx& c) {
+        if (err != cudaSuccess) return;
+        kern<<<grid, kBlock, 0, st>>>(c);
         launches++;
         note(cudaGetLastError());
     }
-    void fill(void* p, int v, size_t bytes) { note(cudaMemsetAsync(p, v, bytes, st)); }
+    // Everything before the stages (the c of the stages: its sorted keys are
+    // only needed here).
+    void prelude(Ctx& c) {
+        auto blocks = [](long long items) { return (unsigned)((items + kBlock - 1) / kBlock); };
+        if (c.n <= kRankPoints) {
+            launch(gcdt_rank_keys, dim3(blocks(c.n + 1ll)), c);
+            if (c.n > 0) launch(gcdt_rank, dim3(blocks(c.n), (c.n + kRankTile - 1) / kRankTile), c);
+            launch(gcdt_rank_points, dim3(blocks(c.n + 4ll)), c);
+            if (c.n > 0 || c.s > 0) launch(gcdt_rank_check, dim3(blocks(c.n > c.s ? c.n : c.s)), c);
+            return;
+        }
+        note(cudaMemsetAsync(c.cnt, 0, sizeof(Counters), st));
+        launch(gcdt_keys, dim3(blocks(c.n)), c);
+        sort(c, c.n);
+        launch(gcdt_points, dim3(blocks(c.n + 4ll)), c);
+        if (c.s > 0) launch(gcdt_segments, dim3(blocks(c.s)), c);
+    }
     // All rounds run in one cooperative launch sized to the co-resident
     // block count, so every block is resident and the grid barrier is safe.
     int grid_limit = 0;   // at most this many blocks (0: no limit)
@@ -338,10 +416,12 @@ gcdt_status enqueue(gcdt_context* ctx, const int32_t* d_points, int32_t n, const
     bk.profile = ctx->profile != 0;
     bk.ev_stage0 = ctx->evs0;
     bk.ev_stage1 = ctx->evs1;
-    bk.note(cudaEventRecord(ctx->evs0, bk.st));   // both stage events exist even if the launch is skipped
-    bk.note(cudaEventRecord(ctx->evs1, bk.st));
     bk.note(cudaEventRecord(ctx->ev0, bk.st));
     enqueue_solve(bk, c);
+    if (bk.err != cudaSuccess) {                   // no stage launch: its events exist all the same
+        cudaEventRecord(ctx->evs0, bk.st);
+        cudaEventRecord(ctx->evs1, bk.st);
+    }
     bk.note(cudaMemcpyAsync(ctx->hcnt, c.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, bk.st));
     bk.note(cudaEventRecord(ctx->ev1, bk.st));
     ctx->pending = true;

@@ -372,9 +372,12 @@ GCDT_HD unsigned long long hilbert60(int2 p) {
 // order (headline solve 28.20 -> 27.88 ms, 305 -> 267 flip sub-rounds).
 GCDT_HD unsigned long long sort_key60(int2 p) { return GCDT_SORT_CURVE ? hilbert60(p) : morton60(p); }
 
+GCDT_HD void check_range(const Ctx& c, int2 p) {
+    if (p.x < 1 || p.y < 1 || p.x > kBoxMax - 1 || p.y > kBoxMax - 1) fail(c, ST_BAD_INPUT);
+}
 GCDT_HD void body_keys(const Ctx& c, int i) {
     int2 p = c.in_xy[i];
-    if (p.x < 1 || p.y < 1 || p.x > kBoxMax - 1 || p.y > kBoxMax - 1) fail(c, ST_BAD_INPUT);
+    check_range(c, p);
     c.keys[i] = sort_key60(p);
     c.vals[i] = i;
 }

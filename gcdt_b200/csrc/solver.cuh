@@ -400,24 +400,35 @@ GCDT_HD int run_stages(EX& ex, Ctx c) {
 // segment set-up, then hand over to the stages (one persistent kernel on the
 // GPU).  Everything is enqueued on the backend's stream without waiting:
 // errors found by the set-up kernels make the stage kernel stop at once.
+// A backend with a prelude of its own (fewer, fused launches) does all of it
+// but the stages.
+template <class BK, class = void>
+struct HasPrelude { static constexpr bool value = false; };
+template <class BK>
+struct HasPrelude<BK, decltype((void)&BK::prelude)> { static constexpr bool value = true; };
+
 template <class BK>
 void enqueue_solve(BK& bk, Ctx c) {
-    const int n = c.n;
-    const long long T = c.ntri;
-    bk.fill(c.cnt, 0, sizeof(Counters));
-    bk.fill(c.vote, 0, 8 * T);
-    bk.fill(c.claim, 0, 8 * T);
-    bk.fill(c.qst, 0, 4 * T);
-    if (n > 0) {
-        bk.launch(K_KEYS, c, n);
-        bk.sort(c, n);
-    }
-    bk.launch(K_GATHER, c, n + 4);
-    bk.launch(K_ROOT, c, 1);
-    if (n > 0) bk.launch(K_LEVEL, c, n);
-    if (c.s > 0) {
-        bk.launch(K_SEG_INIT, c, c.s);
-        bk.launch(K_SEG_LEVEL0, c, c.s);
+    if constexpr (HasPrelude<BK>::value) {
+        bk.prelude(c);
+    } else {
+        const int n = c.n;
+        const long long T = c.ntri;
+        bk.fill(c.cnt, 0, sizeof(Counters));
+        bk.fill(c.vote, 0, 8 * T);
+        bk.fill(c.claim, 0, 8 * T);
+        bk.fill(c.qst, 0, 4 * T);
+        if (n > 0) {
+            bk.launch(K_KEYS, c, n);
+            bk.sort(c, n);
+        }
+        bk.launch(K_GATHER, c, n + 4);
+        bk.launch(K_ROOT, c, 1);
+        if (n > 0) bk.launch(K_LEVEL, c, n);
+        if (c.s > 0) {
+            bk.launch(K_SEG_INIT, c, c.s);
+            bk.launch(K_SEG_LEVEL0, c, c.s);
+        }
     }
     bk.stages(c);
 }

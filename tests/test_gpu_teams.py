@@ -44,7 +44,8 @@ def _equal(got, want):
 
 # one block's list capacity is 512, the tails' default threshold 1,024; a
 # cluster solves up to 15,000 points
-@pytest.mark.parametrize("n", [1, 2, 3, 64, 480, 512, 513, 1024, 1025, 4000, 14800, 14999, 15000, 15001, 40000])
+@pytest.mark.parametrize("n", [1, 2, 3, 64, 480, 512, 513, 1024, 1025, 4000, 14800, 14999, 15000, 15001, 16383, 16384, 16385,
+                               40000])
 def test_single_solve_has_the_host_bytes(n):
     xy, cons = _instance(n, 3 * n)
     if n > 14000:       # exact point counts on both sides of the cluster's limit
@@ -97,3 +98,33 @@ def test_batch_of_mixed_cluster_sizes():
     for i in (0, 1, 2, 7, 8, 37, 38, 97, 98, 397, 398, 497):
         xy, cons = inst[i]
         assert _equal(res[i], _host(xy, cons, (2, 16, 1, 1, 0, 1024, 1024))), (i, len(xy))
+
+
+@pytest.mark.parametrize("n", [2, 1023, 1024, 1025, 16384, 16385])
+def test_set_up_refuses_bad_points_at_every_size(n):
+    """The set-up that compares all pairs of keys (up to 16,384 points, in
+    tiles of 1,024) and the one that sorts refuse the same inputs: two equal
+    points wherever they are, and a coordinate on or outside the box."""
+    rng = np.random.default_rng(n)
+    xy = np.unique(rng.integers(1, 1 << 29, size=(n + 64, 2)), axis=0).astype(np.int32)
+    xy = rng.permutation(xy)[:n]
+    tri = g.Triangulator(n, 1)
+
+    def status(pts):
+        try:
+            tri.triangulate_host(pts)
+        except g.GcdtError as e:
+            return e.status
+        return "OK"
+
+    assert status(xy) == "OK"
+    for i, j in ((0, n - 1), (n // 2, n // 2 + 1 if n > 2 else 0)):
+        bad = xy.copy()
+        bad[i] = bad[j]
+        assert status(bad) == "BAD_INPUT"
+    for value in (0, -5, (1 << 30) - 1):
+        bad = xy.copy()
+        bad[n - 1, 1] = value
+        assert status(bad) == "BAD_INPUT"
+    assert status(xy) == "OK"
+    tri.close()
