@@ -417,7 +417,15 @@ template <int K, class SH>
 __device__ __forceinline__ void round_items(const SH& sh) {
     const Ctx c = items_view(sh.ctx, K);
     const int count = (int)sh.count, stride = blockDim.x - 32;
-    for (int i = threadIdx.x; i < count; i += stride) dispatch(K, c, i);
+    for (int i = threadIdx.x; i < count; i += stride) {
+        if constexpr (K == K_FLIP_FIX) {        // its loads side by side (body_flip_fix: edge by edge)
+            const int ks[1] = {i};
+            const int2 f[1] = {flip_first(c, FP_FIX, i)};
+            flip_fix_multi_f<1>(c, ks, f);
+        } else {
+            dispatch(K, c, i);
+        }
+    }
 }
 
 // A worker's share of a published single-block phase or command.

@@ -445,12 +445,13 @@ GCDT_HD long long dot3(int2 a, int2 u, int2 b) {  // (u-a).(b-a)
 GCDT_HD int locate_from_vertex(const Ctx& c, int a, int t, int2 p) {
     for (int restart = 0; restart < 4096; ++restart) {
         int2 pa = c.P[a];
-        int t0 = t, found = -1, fslot = 0, u = -1, w = -1;
+        int t0 = t, found = -1;             // found: the edge the line leaves by, seen from beyond
+        int2 pu, pw;                        // its ends
         for (int g = 0; g < 4096; ++g) {
-            int4 tv = tri_v(c, t);
+            const int4 tv = tri_v(c, t), ta = tri_a(c, t);
             int i = slot_of(tv, a), i1 = nx3(i), i2 = nx3(i1);
-            u = comp(tv, i1); w = comp(tv, i2);
-            int2 pu = c.P[u], pw = c.P[w];
+            const int u = comp(tv, i1), w = comp(tv, i2);
+            pu = c.P[u]; pw = c.P[w];
             int ou = orient2d(pa, pu, p), ow = orient2d(pa, pw, p);
             if (ou == 0 && dot3(pa, pu, p) > 0) {
                 if (dot3(pa, p, pu) > dot3(pa, p, p)) return t;   // p inside edge (a,u)
@@ -462,29 +463,26 @@ GCDT_HD int locate_from_vertex(const Ctx& c, int a, int t, int2 p) {
             }
             if (ou > 0 && ow < 0) {
                 if (orient2d(pu, pw, p) >= 0) return t;
-                found = t; fslot = i; break;
+                found = comp(ta, i); break;
             }
-            int nb = comp(tri_a(c, t), i2);
+            int nb = comp(ta, i2);
             if (nb < 0) return -1;
             t = nb >> 2;
             if (t == t0) return -1;
         }
         if (found == -2) continue;          // t contains the new a
-        if (found < 0) return -1;
-        int cur = found, cs = fslot;
-        int next_a = -1;
+        int en = found, next_a = -1;
         for (int steps = 0; steps < (1 << 22); ++steps) {
-            int en = comp(tri_a(c, cur), cs);
             if (en < 0) return -1;
             int n = en >> 2, j = en & 3;
-            int x = comp(tri_v(c, n), j);
+            const int4 nv = tri_v(c, n), na = tri_a(c, n);
+            int x = comp(nv, j);
             int2 px = c.P[x];
             // n = (x, w, u): p is inside iff it is left of (u,x) and (x,w)
-            if (orient2d(c.P[u], px, p) >= 0 && orient2d(px, c.P[w], p) >= 0) return n;
+            if (orient2d(pu, px, p) >= 0 && orient2d(px, pw, p) >= 0) return n;
             int ox = orient2d(pa, p, px);
             if (ox == 0) { next_a = x; t = n; break; }
-            cur = n;
-            if (ox < 0) { u = x; cs = nx3(nx3(j)); } else { w = x; cs = nx3(j); }
+            if (ox < 0) { pu = px; en = comp(na, nx3(nx3(j))); } else { pw = px; en = comp(na, nx3(j)); }
         }
         if (next_a < 0) return -1;
         a = next_a;
@@ -556,7 +554,7 @@ GCDT_HD void body_vt_live(const Ctx& c, int k) {
 // vertex, so it lies on at most one edge).
 GCDT_HD int walk(const Ctx& c, int t, int2 p, int limit, int* edge) {
     for (int it = 0; it < limit; ++it) {
-        int4 tv = tri_v(c, t);
+        const int4 tv = tri_v(c, t), ta = tri_a(c, t);
         int2 a = c.P[tv.x], b = c.P[tv.y], cc = c.P[tv.z];
         int side = -1, zero = -1;
         int r = it % 3;
@@ -567,7 +565,7 @@ GCDT_HD int walk(const Ctx& c, int t, int2 p, int limit, int* edge) {
             else if (o == 0) zero = s;
         }
         if (side < 0) { *edge = zero; return t; }
-        int nb = comp(tri_a(c, t), side);
+        int nb = comp(ta, side);
         if (nb < 0) return -1;
         t = nb >> 2;
     }
@@ -731,21 +729,35 @@ GCDT_HD int qtri(int e) { return (int)((unsigned)e >> 3); }
 // The children of the inserted points are distinct triangles, so the first
 // flip queue of a round needs no de-duplication.
 
-// The edge in slot s of split child ch names its old neighbour: point it at
-// the neighbour's child that holds the edge when the neighbour was split in
-// this round too (its adjacency row's round stamp; flips of the round come
-// after this phase), else write ch into the neighbour's row.  The
-// neighbour's record is the sector the second case writes anyway.
-GCDT_HD void resolve_split_edge(const Ctx& c, int ch, int s) {
-    int4* row = &tri_a(c, ch);
-    int old = comp(*row, s);
-    if (old < 0) return;
-    int m = old >> 2, ms = old & 3;
-    const int4 mv = tri_v(c, m), ma = tri_a(c, m);
-    if (ma.w == (int)c.round) {
-        ((int*)row)[s] = enc(split_child(tri_v(c, ch), s, mv, m, ms), ms);
-    } else {
-        ((int*)&tri_a(c, m))[ms] = enc(ch, s);
+// The old edges of a split's children, for one inserted point: the edge in
+// slot s of child ch names its old neighbour; point it at the neighbour's
+// child that holds the edge when the neighbour was split in this round too
+// (its adjacency row's round stamp; flips of the round come after this
+// phase), else write ch into the neighbour's row.  The neighbour's record is
+// the sector the second case writes anyway.  All loads come before the first
+// write (they read no word that this phase writes), so that the three or four
+// edges' chains run side by side instead of one after the other.
+template <int E>
+GCDT_HD void resolve_split_edges(const Ctx& c, const int (&ch)[E], const int (&s)[E]) {
+    int old[E];
+    int4 cv[E], mv[E];
+    int mr[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        old[k] = ((const int*)&tri_a(c, ch[k]))[s[k]];
+        cv[k] = tri_v(c, ch[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        mv[k] = old[k] >= 0 ? tri_v(c, old[k] >> 2) : make_int4(0, 0, 0, 0);
+        mr[k] = old[k] >= 0 ? tri_a(c, old[k] >> 2).w : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        if (old[k] < 0) continue;
+        const int m = old[k] >> 2, ms = old[k] & 3;
+        if (mr[k] == (int)c.round) ((int*)&tri_a(c, ch[k]))[s[k]] = enc(split_child(cv[k], s[k], mv[k], m, ms), ms);
+        else ((int*)&tri_a(c, m))[ms] = enc(ch[k], s[k]);
     }
 }
 
@@ -761,9 +773,8 @@ GCDT_HD int fix_winner(const Ctx& c, int2 w, int4& qe) {
     // so the circle through q and the spoke's far edge excludes the third
     // corner; on an edge split the spoke's quadrilateral is not even convex).
     if (code == 7) {
-        resolve_split_edge(c, t, 0);
-        resolve_split_edge(c, T1, 1);
-        resolve_split_edge(c, T2, 2);
+        const int ch[3] = {t, T1, T2}, sl[3] = {0, 1, 2};
+        resolve_split_edges<3>(c, ch, sl);
         qe = make_int4(qentry(t, 1), qentry(T1, 2), qentry(T2, 4), 0);
         return 3;
     }
@@ -772,10 +783,8 @@ GCDT_HD int fix_winner(const Ctx& c, int2 w, int4& qe) {
     int en = comp(tri_a(c, T1), e);     // A2 slot e = enc(B1, e2)
     int n = en >> 2, e2 = en & 3;
     int f1 = nx3(e2), f2 = nx3(f1);
-    resolve_split_edge(c, t, e1);
-    resolve_split_edge(c, T1, e_2);
-    resolve_split_edge(c, n, f1);
-    resolve_split_edge(c, T2, f2);
+    const int ch[4] = {t, T1, n, T2}, sl[4] = {e1, e_2, f1, f2};
+    resolve_split_edges<4>(c, ch, sl);
     // outer edge and the half of the split edge
     qe = make_int4(qentry(t, (1 << e1) | (1 << e)), qentry(T1, (1 << e_2) | (1 << e)),
                    qentry(n, (1 << f1) | (1 << e2)), qentry(T2, (1 << f2) | (1 << e2)));
