@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kClusterThreads, 2) gcdt_batch_cluster(BatchAr
     }
     Ctx c = sh.ctx;
     TeamExec<true, SH> ex{cnt, rank, size, &sh};
-    ex.take_snapshot();
+    ex.start();
     const int st = solve_instance(ex, c);
     if (rank == 0 && threadIdx.x == kWork) a.desc[inst].status = st;
     publish(sh, kExit, c, 0, false);

@@ -614,6 +614,12 @@ struct TeamExec {
     // word k in lane k, read right after each barrier.
     unsigned long long snap = 0;
     unsigned parity = 0;                     // of the grid barriers passed, in the top bit
+    // Before the first phase.  (The counter's top bit cannot change before
+    // this block has arrived at a barrier.)
+    __device__ void start() {
+        parity = *(volatile unsigned*)&cnt->bar_count & 0x80000000u;
+        take_snapshot();
+    }
 
     __device__ int narrow_flips(Ctx& c, Driver& D, long long& nq);
     __device__ int narrow_rounds(Ctx& c, Driver& D, long long nact);
@@ -629,7 +635,7 @@ struct TeamExec {
     // every block has arrived, and a block waits for the top bit to reach
     // the barrier's parity, which its driver counts along.  One atomic per
     // block, whose result nobody waits for, and no reset.  The counter starts
-    // each launch at 0 (the solve clears its counters).  Every wait is
+    // each solve at 0 (it clears its counters).  Every wait is
     // bounded: after spin_limit polls (2^25, about ten seconds, in a solve)
     // the block records ST_BARRIER and stops waiting, and once that bit is
     // set no block waits or works any more, so the kernel always ends.  A

@@ -25,14 +25,14 @@ __global__ void __launch_bounds__(kBlock) gcdt_keys(Ctx c) {
 __global__ void __launch_bounds__(kBlock) gcdt_points(Ctx c) {
     const int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= c.n + 4) return;
-    body_gather(c, i);
+    body_gather<false>(c, i);
     if (i < c.n) body_level(c, i);
     if (i == 0) body_root(c, 0);
 }
 __global__ void __launch_bounds__(kBlock) gcdt_segments(Ctx c) {
     const int k = blockIdx.x * kBlock + threadIdx.x;
     if (k >= c.s) return;
-    body_seg_init(c, k);
+    body_seg_init<false>(c, k);
     body_seg_level0(c, k);
 }
 
@@ -121,7 +121,7 @@ struct ParamView {
 // kCluster: the launch is one thread-block cluster (a small problem), and its
 // phases end with the cluster barrier.
 template <bool kProf, bool kCluster>
-__global__ void __launch_bounds__(kPersistBlock, 1) gcdt_stages(const __grid_constant__ Ctx c) {
+__global__ void __launch_bounds__(kPersistBlock, 1) gcdt_stages(const __grid_constant__ Ctx c, int part) {
     __shared__ StageShared sh;
     {
         const int* src = reinterpret_cast<const int*>(&c);
@@ -132,13 +132,53 @@ __global__ void __launch_bounds__(kPersistBlock, 1) gcdt_stages(const __grid_con
     if (threadIdx.x >= 32 * kStageWorkers) {
         TeamExec<kCluster, StageShared> ex{c.cnt, blockIdx.x, gridDim.x, &sh};
         ex.prof = kProf;
-        ex.take_snapshot();
-        run_stages(ex, c);
+        ex.start();
+        run_stages(ex, c, part);
         publish(sh, kExit, c, 0, false);
         block_sync(kBarWork);
     } else {
         team_worker<kCluster, 2>(sh, blockIdx.x, gridDim.x, ParamView{c, sh.ctx});
     }
+}
+
+// Phases of a large solve that run as launches of their own between the
+// stage kernel's parts: a walk per point, a few atomics per triangle and a
+// copy need 30 to 46 registers, so that twice the stage kernel's warps are in
+// flight (10.2M points: activations 1.45 -> 0.91 ms, maps 0.50 -> 0.16,
+// output 0.33 -> 0.20).  The activation casts the first round's votes too.
+__device__ __forceinline__ bool solve_failed(const Ctx& c) { return (c.cnt->status | c.cnt->err[0] | c.cnt->err[1]) != 0; }
+__global__ void __launch_bounds__(kBlock) gcdt_vt_reset(Ctx c) {
+    const int v = blockIdx.x * kBlock + threadIdx.x;
+    if (v < c.n + 4) body_vt_reset(c, v);
+}
+__global__ void __launch_bounds__(kBlock) gcdt_vt_live(Ctx c, int level) {
+    const int k = blockIdx.x * kBlock + threadIdx.x;
+    c.level = level;
+    if (k < c.n + 2 && !solve_failed(c)) body_vt_live(c, k);
+}
+__global__ void __launch_bounds__(kBlock) gcdt_activate(Ctx c, int level) {
+    const int i = blockIdx.x * kBlock + threadIdx.x;
+    if (i >= c.n || solve_failed(c)) return;
+    c.level = level;
+    // the list and its cursor, from the driver state of the part before
+    c.act_next = reinterpret_cast<int*>(c.cnt->handoff[offsetof(Driver, actA) / 8]);
+    c.base_act = c.cnt->handoff[offsetof(Driver, e_act0) / 8];
+    c.round = reinterpret_cast<const unsigned*>(c.cnt->handoff)[offsetof(Driver, round) / 4] + 1;
+    if (c.lvl[i] != level) return;
+    const int2 p = c.P[i];
+    const int t = activate_location(c, i, p);
+    if (t < 0) { fail(c, ST_ITER_LIMIT); return; }
+    // what the relocation of the level's first round does with a point that
+    // is in its triangle already
+    const int e = edge_of(c, t, p);
+    c.loc[i] = t;
+    c.pedge[i] = (signed char)e;
+    c.act_next[append_slot(&c.cnt->cur_act0, c.base_act)] = i;
+    cast_votes(c, i, t, e);
+}
+__global__ void __launch_bounds__(kBlock) gcdt_output(Ctx c) {
+    const int t = blockIdx.x * kBlock + threadIdx.x;
+    if (t < c.ntri && !solve_failed(c)) body_output(c, t);
 }
 
 // Failure-detection probe of the grid barrier: every block but `absent`
@@ -173,16 +213,17 @@ struct DeviceBackend {
 
     void note(cudaError_t e) { if (e != cudaSuccess && err == cudaSuccess) err = e; }
 
-    void launch(void (*kern)(Ctx), dim3 grid, const Ctx& c) {
+    template <class... A>
+    void launch(void (*kern)(Ctx, A...), dim3 grid, const Ctx& c, A... args) {
         if (err != cudaSuccess) return;
-        kern<<<grid, kBlock, 0, st>>>(c);
+        kern<<<grid, kBlock, 0, st>>>(c, args...);
         launches++;
         note(cudaGetLastError());
     }
+    static unsigned blocks(long long items) { return (unsigned)((items + kBlock - 1) / kBlock); }
     // Everything before the stages (the c of the stages: its sorted keys are
     // only needed here).
     void prelude(Ctx& c) {
-        auto blocks = [](long long items) { return (unsigned)((items + kBlock - 1) / kBlock); };
         if (c.n <= kRankPoints) {
             launch(gcdt_rank_keys, dim3(blocks(c.n + 1ll)), c);
             if (c.n > 0) launch(gcdt_rank, dim3(blocks(c.n), (c.n + kRankTile - 1) / kRankTile), c);
@@ -204,7 +245,8 @@ struct DeviceBackend {
     void stages(const Ctx& c) {
         if (err != cudaSuccess) return;
         Ctx cc = c;
-        void* args[] = {&cc};
+        int part = -1;
+        void* args[] = {&cc, &part};
         if (ev_stage0) note(cudaEventRecord(ev_stage0, st));
         const int cluster = cluster_blocks(c.n);
         if (cluster > 0) {
@@ -220,6 +262,7 @@ struct DeviceBackend {
             cfg.attrs = at;
             cfg.numAttrs = 1;
             note(cudaLaunchKernelExC(&cfg, kern, args));
+            launches++;
         } else {
             int dev = 0, sms = 0, per_sm = 0;
             note(cudaGetDevice(&dev));
@@ -227,13 +270,31 @@ struct DeviceBackend {
             const void* kern = profile ? (const void*)gcdt_stages<true, false> : (const void*)gcdt_stages<false, false>;
             note(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPersistBlock, 0));
             if (err != cudaSuccess || sms <= 0 || per_sm <= 0) { note(cudaErrorLaunchOutOfResources); return; }
-            int blocks = sms * per_sm;
-            if (grid_limit > 0 && grid_limit < blocks) blocks = grid_limit;
-            note(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kPersistBlock), args, 0, st));
+            int nblocks = sms * per_sm;
+            if (grid_limit > 0 && grid_limit < nblocks) nblocks = grid_limit;
+            const dim3 grid(nblocks);
+            if (c.n < kSplitPoints || profile) {
+                note(cudaLaunchCooperativeKernel(kern, grid, dim3(kPersistBlock), args, 0, st));
+                launches++;
+            } else {
+                for (part = 0; part < c.nlevels; ++part) {
+                    if (part > 0) {
+                        launch(gcdt_vt_reset, dim3(blocks(c.n + 4ll)), c);
+                        launch(gcdt_vt_live, dim3(blocks(c.n + 2ll)), c, part);
+                        launch(gcdt_activate, dim3(blocks(c.n)), c, part);
+                    }
+                    if (err != cudaSuccess) return;
+                    note(cudaLaunchCooperativeKernel(kern, grid, dim3(kPersistBlock), args, 0, st));
+                    launches++;
+                }
+                launch(gcdt_output, dim3(blocks(c.ntri)), c);
+            }
         }
         if (ev_stage1) note(cudaEventRecord(ev_stage1, st));
-        launches++;
     }
+    // From here on the launches' gaps cost less than the phases gain (300,000
+    // points: 2.40 -> 2.37 ms, 1M 3.96 -> 3.88, 10.2M 21.4 -> 20.3).
+    static constexpr int kSplitPoints = 200000;
     // Blocks of the cluster that solves n points, 0: the whole grid does.  A
     // small problem's phases are shorter than the grid barrier: eight blocks
     // (the portable cluster size) with the cluster barrier take 0.90 ms

@@ -382,14 +382,16 @@ GCDT_HD void body_keys(const Ctx& c, int i) {
     c.vals[i] = i;
 }
 
-// After the sort (sorted keys/vals in keys/vals): gather points, permutation,
-// inverse permutation; adjacent equal keys are duplicate points.
+// After the sort (sorted keys/vals in keys/vals): gather points, permutation
+// and, where segments are looked up in it, inverse permutation; adjacent
+// equal keys are duplicate points.
+template <bool kRank = true>
 GCDT_HD void body_gather(const Ctx& c, int i) {
     if (i < c.n) {
         int j = c.vals[i];
         c.P[i] = c.in_xy[j];
         c.perm[i] = j;
-        c.rank[j] = i;
+        if (kRank) c.rank[j] = i;
         if (i > 0 && c.keys[i] == c.keys[i - 1]) fail(c, ST_BAD_INPUT);
     } else if (i < c.n + 4) {
         int k = i - c.n;
@@ -495,30 +497,30 @@ GCDT_HD int locate_from_vertex(const Ctx& c, int a, int t, int2 p) {
 // (R,0)-(0,R), rawMesh.cu:37-57), otherwise a straight-line walk from the
 // nearer of the previous level's preceding and following points along the
 // sort curve, which are already vertices.
-GCDT_HD void body_activate(const Ctx& c, int i) {
-    if (c.lvl[i] != c.level) return;
-    int t;
+GCDT_HD int activate_location(const Ctx& c, int i, int2 p) {
     if (c.level == 0) {
         int2 rd = make_int2(kBoxMax, 0), lt = make_int2(0, kBoxMax);
-        t = orient2d(rd, lt, c.P[i]) >= 0 ? 0 : 1;
-    } else {
-        // start from the nearer of the two previous-level samples around i
-        // in curve order (both are vertices already)
-        // (no index computed at run time: it would keep a grid phase's whole
-        // view of the context in local memory)
-        const int s = c.level == 1 ? c.stride[0] : (c.level == 2 ? c.stride[1] : c.stride[2]);
-        int sv = i - i % s;
-        const int hi = sv + s;
-        const int2 p = c.P[i];
-        if (hi < c.n) {
-            int2 a = c.P[sv], b = c.P[hi];
-            long long da = (long long)(a.x - p.x) * (a.x - p.x) + (long long)(a.y - p.y) * (a.y - p.y);
-            long long db = (long long)(b.x - p.x) * (b.x - p.x) + (long long)(b.y - p.y) * (b.y - p.y);
-            if (db < da) sv = hi;
-        }
-        t = locate_from_vertex(c, sv, c.vt[sv], p);
-        if (t < 0) { fail(c, ST_ITER_LIMIT); return; }
+        return orient2d(rd, lt, p) >= 0 ? 0 : 1;
     }
+    // start from the nearer of the two previous-level samples around i in
+    // curve order (both are vertices already)
+    // (no index computed at run time: it would keep a grid phase's whole
+    // view of the context in local memory)
+    const int s = c.level == 1 ? c.stride[0] : (c.level == 2 ? c.stride[1] : c.stride[2]);
+    int sv = i - i % s;
+    const int hi = sv + s;
+    if (hi < c.n) {
+        int2 a = c.P[sv], b = c.P[hi];
+        long long da = (long long)(a.x - p.x) * (a.x - p.x) + (long long)(a.y - p.y) * (a.y - p.y);
+        long long db = (long long)(b.x - p.x) * (b.x - p.x) + (long long)(b.y - p.y) * (b.y - p.y);
+        if (db < da) sv = hi;
+    }
+    return locate_from_vertex(c, sv, c.vt[sv], p);
+}
+GCDT_HD void body_activate(const Ctx& c, int i) {
+    if (c.lvl[i] != c.level) return;
+    const int t = activate_location(c, i, c.P[i]);
+    if (t < 0) { fail(c, ST_ITER_LIMIT); return; }
     c.loc[i] = t;
     c.act_next[append_slot(&c.cnt->cur_act0, c.base_act)] = i;
 }
@@ -1175,14 +1177,28 @@ GCDT_HD void body_flip_fix_pair(const Ctx& c, int k0, int k1) {
 
 // ---------------------------------------------------------------- constraints
 
+// Sorted position of input point j: its key's place among the sorted keys
+// (distinct, or the solve stops).
+GCDT_HD int rank_by_key(const Ctx& c, int j) {
+    const unsigned long long key = sort_key60(c.in_xy[j]);
+    int lo = 0, hi = c.n;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (c.keys[mid] <= key) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
 // Map segment endpoints to sorted ids; reject malformed segments.
+template <bool kRank = true>
 GCDT_HD void body_seg_init(const Ctx& c, int k) {
     int2 ab = c.in_cons[k];
     if (ab.x < 0 || ab.y < 0 || ab.x >= c.n || ab.y >= c.n || ab.x == ab.y) {
         fail(c, ST_BAD_INPUT);
         c.seg[k] = make_int4(0, 0, 0, 0);   // .z != -1: not a valid segment
     } else {
-        c.seg[k] = make_int4(c.rank[ab.x], c.rank[ab.y], -1, 0);
+        c.seg[k] = kRank ? make_int4(c.rank[ab.x], c.rank[ab.y], -1, 0)
+                         : make_int4(rank_by_key(c, ab.x), rank_by_key(c, ab.y), -1, 0);
     }
     c.pend[k] = k;
 }

@@ -247,8 +247,10 @@ GCDT_HD int flip_until_delaunay(EX& ex, Ctx& c, Driver& D, long long nq) {
     return flip_loop(ex, c, D, nq, (long long)1 << 62);
 }
 
+// Rounds until the nact active points are inserted.  voted: their votes for
+// the first round are cast already (by the launch that activated them).
 template <class EX>
-GCDT_HD int insert_rounds(EX& ex, Ctx& c, Driver& D, long long nact) {
+GCDT_HD int insert_rounds(EX& ex, Ctx& c, Driver& D, long long nact, bool voted = false) {
     while (nact > 0) {
         if (EX::kCanNarrow && nact <= c.narrow_act) {
             // the single-block tail starts from a Delaunay mesh: the carried
@@ -278,13 +280,16 @@ GCDT_HD int insert_rounds(EX& ex, Ctx& c, Driver& D, long long nact) {
                 continue;
             }
         }
-        c.act = D.actA; c.act_next = D.actB;
-        c.base_act = D.e_act;
-        run_phase(ex, c, D, K_RELOC_VOTE, nact);
-        D.e_act = ex.cursor(&c.cnt->cur_act);
-        if (D.errs) return D.errs;
-        nact = (long long)(D.e_act - c.base_act);
-        { int* t = D.actA; D.actA = D.actB; D.actB = t; }
+        if (!voted) {
+            c.act = D.actA; c.act_next = D.actB;
+            c.base_act = D.e_act;
+            run_phase(ex, c, D, K_RELOC_VOTE, nact);
+            D.e_act = ex.cursor(&c.cnt->cur_act);
+            if (D.errs) return D.errs;
+            nact = (long long)(D.e_act - c.base_act);
+            int* t = D.actA; D.actA = D.actB; D.actB = t;
+        }
+        voted = false;
         if (nact == 0) break;
         c.act = D.actA; c.act_next = D.actB;
         c.base_win = D.e_win;
@@ -358,8 +363,12 @@ GCDT_HD int insert_constraints(EX& ex, Ctx& c, Driver& D) {
 
 // Everything after the sort: the insertion levels, the constraint stage
 // after level 0, and the output.  Cursors start at 0 (cleared by the host).
+// part >= 0: only level `part`, for a solve whose vertex -> triangle maps,
+// activations with the first round's votes (from level 1 on) and output run
+// as launches of their own; the driver state then goes from part to part
+// through the hand-off area.
 template <class EX>
-GCDT_HD int run_stages(EX& ex, Ctx c) {
+GCDT_HD int run_stages(EX& ex, Ctx c, int part = -1) {
     const int n = c.n;
     Driver D;
     D.actA = c.act; D.actB = c.act_next; D.qa = c.queue; D.qb = c.queue_next;
@@ -367,32 +376,38 @@ GCDT_HD int run_stages(EX& ex, Ctx c) {
     D.round = 0; D.sr = 0; D.rounds = 0; D.subrounds = 0; D.crounds = 0;
     D.e_act0 = D.e_act = D.e_win = D.e_q = D.e_flip = D.e_pend = D.e_law = D.e_scr = 0;
     D.nphase = 0; D.errs = 0;
-    // set-up (keys, gather, segments) flagged bad input: stop before any phase
+    // set-up (keys, gather, segments) flagged bad input, or an earlier part
+    // ended with an error: stop before any phase
     if (ex.word(&c.cnt->status) | ex.word(&c.cnt->err[0]) | ex.word(&c.cnt->err[1])) {
-        ex.finish(c, 0, 0, 0, 0);
+        if (part <= 0) ex.finish(c, 0, 0, 0, 0);
         return ST_BAD_INPUT;
     }
+    if (part > 0) load_driver(c.cnt, D);
     int rc = 0;
-    for (int l = 0; l < c.nlevels && n > 0 && rc == 0; ++l) {
+    const int end = part < 0 ? c.nlevels : part + 1;
+    for (int l = part < 0 ? 0 : part; l < end && n > 0 && rc == 0; ++l) {
         c.level = l;
-        if (l > 0) {
-            run_phase(ex, c, D, K_VT_RESET, n + 4);
-            run_phase(ex, c, D, K_VT_LIVE, n + 2);
-        }
         c.act_next = D.actA;
         c.base_act = D.e_act0;
-        run_phase(ex, c, D, K_ACTIVATE, n);
+        if (part <= 0) {
+            if (l > 0) {
+                run_phase(ex, c, D, K_VT_RESET, n + 4);
+                run_phase(ex, c, D, K_VT_LIVE, n + 2);
+            }
+            run_phase(ex, c, D, K_ACTIVATE, n);
+        }
         D.e_act0 = ex.cursor(&c.cnt->cur_act0);
         if ((rc = D.errs)) break;
-        rc = insert_rounds(ex, c, D, (long long)(D.e_act0 - c.base_act));
+        rc = insert_rounds(ex, c, D, (long long)(D.e_act0 - c.base_act), part > 0);
         if (rc == 0 && l == 0 && c.s > 0) rc = insert_constraints(ex, c, D);
     }
     if (rc == 0 && n == 0 && c.s > 0) rc = ST_BAD_INPUT;
-    if (rc == 0) {
+    if (rc == 0 && part < 0) {
         run_phase(ex, c, D, K_OUTPUT, c.ntri);
         rc = D.errs;
     }
     ex.finish(c, D.rounds, D.subrounds, D.crounds, rc | D.errs);
+    if (part >= 0) save_driver(c.cnt, D);       // (every block's driver: the same words)
     return rc;
 }
 

@@ -128,3 +128,39 @@ def test_set_up_refuses_bad_points_at_every_size(n):
         assert status(bad) == "BAD_INPUT"
     assert status(xy) == "OK"
     tri.close()
+
+
+@pytest.mark.parametrize("extra,levels", [(-1, (3, 512, 8)), (0, (3, 512, 8)), (1, (1, 1, 1)), (1, (2, 64, 1)),
+                                          (1, (4, 1024, 64))])
+def test_solve_in_parts_has_the_host_bytes(extra, levels):
+    """From 200,000 points on, the levels' activations (with the first
+    round's votes), the maps and the output are launches of their own: both
+    sides of the limit, every number of parts, with segments."""
+    xy, cons = g.generate(g.GEN_SCALE, 11, 200000, 6, 30)
+    drop = len(xy) - (200000 + extra)
+    used = np.zeros(len(xy), bool)
+    used[cons.reshape(-1)] = True
+    keep = np.ones(len(xy), bool)
+    keep[np.flatnonzero(~used)[:drop]] = False
+    new = np.cumsum(keep) - 1
+    xy, cons = np.ascontiguousarray(xy[keep]), np.ascontiguousarray(new[cons].astype(np.int32))
+    assert len(xy) == 200000 + extra
+    n, s0, s1 = levels
+    strides = (s0, s1, 8 if n == 4 else 1)
+    tri = g.Triangulator(len(xy), len(cons))
+    tri.set_tuning(levels=n, level_stride=strides[:n - 1] or None)
+    got = tri.triangulate_host(xy, cons)
+    assert _equal(got, _host(xy, cons, (n, *strides, 1 << 22, 1024, 1024)))
+    # a budget that runs out in a part ends the solve; the next one is whole
+    tri.set_limits(insertion_rounds=3)
+    with pytest.raises(g.GcdtError) as e:
+        tri.triangulate_host(xy, cons)
+    assert e.value.status == "ITER_LIMIT"
+    tri.set_limits()
+    assert _equal(tri.triangulate_host(xy, cons), got)
+    # crossing segments, found in the first part
+    far = np.argsort(xy.sum(1).astype(np.int64))[[0, -1]], np.argsort(xy[:, 0].astype(np.int64) - xy[:, 1])[[0, -1]]
+    with pytest.raises(g.GcdtError) as e:
+        tri.triangulate_host(xy, np.array(far, np.int32))
+    assert e.value.status == "CONSTRAINT_FAIL"
+    tri.close()
