@@ -90,6 +90,7 @@ struct BlockShared {
     int2 winners[CAP];
     // the fast commands' lists (see fast_flips, fast_round)
     int budget;                 // flip sub-rounds they may take
+    int checked;                // the first one's candidates are in cand
     int tally[3][2];            // flips and losers of a sub-round, in turn of three
     int n_alive, n_won, n_next; // active points, inserted points and survivors of a round
     int n_queue;                // entries of the flip queue they leave
@@ -119,7 +120,7 @@ __device__ __forceinline__ void publish(SH& sh, int k, const Ctx& c, long long c
         } else if (k == kFastFlips) {
             v.queue = c.queue; v.carry_n = c.carry_n;
         } else if (k == K_RELOC_VOTE || k == K_SPLIT || k == K_FIX || k == kFastRound) {
-            v.act = c.act; v.act_next = c.act_next; v.queue_next = c.queue_next; v.winners = c.winners;
+            v.act = c.act; v.act_next = c.act_next; v.queue_next = c.queue_next; v.winners = c.winners; v.cand = c.cand;
             v.base_act = c.base_act; v.base_win = c.base_win; v.base_q = c.base_q;
         } else {
             v.level = c.level; v.lawson_sr = c.lawson_sr;
@@ -138,6 +139,7 @@ template <class SH>
 struct BlockExecT {
     static constexpr bool kCanNarrow = false;
     static constexpr int kFastItems = SH::kCap;
+    static constexpr bool kFixChecks = true;
     SH& sh;
     int2* const all_cand;       // the lists' arrays
     int2* const all_winners;
@@ -146,6 +148,7 @@ struct BlockExecT {
     int2* cur_win = nullptr;
     int2* cur_cand = nullptr;
     int* nxt_q = nullptr;
+    bool checked = false;       // fast_round has left the queue's candidates in sh.cand
 
     __device__ BlockExecT(SH& s, const Ctx& c) : sh(s), all_cand(c.cand), all_winners(c.winners) {}
     // The block's counters, at the driver's cursors.
@@ -161,6 +164,7 @@ struct BlockExecT {
     }
     __device__ void phase(int k, const Ctx& cd, long long count) {
         Ctx c = cd;
+        checked = false;
         const bool fits = count <= SH::kCap;
         c.cand = all_cand; c.winners = all_winners;
         switch (k) {
@@ -179,6 +183,8 @@ struct BlockExecT {
             c.winners = cur_win;
             if (fits) c.queue_next = sh.queue[0];
             cur_q = c.queue_next;
+            cur_cand = 4 * count <= SH::kCap ? sh.cand : c.cand;    // at most four entries each
+            c.cand = cur_cand;
             break;
         case K_FLIP_CHECK:
             c.queue = cur_q;
@@ -211,7 +217,8 @@ struct BlockExecT {
         c.queue = cur_q;
         c.carry_n = (int)D.drop;
         D.drop = 0;
-        if ((threadIdx.x & 31) == 0) sh.budget = (int)left;
+        if ((threadIdx.x & 31) == 0) { sh.budget = (int)left; sh.checked = checked; }
+        checked = false;
         run(kFastFlips, c, nq);
         const int took = sh.subrounds, nf = sh.flips;
         cur_q = sh.queue[(cur_q == sh.queue[0]) ^ ((took + 1) & 1)];
@@ -231,9 +238,11 @@ struct BlockExecT {
         c.act = cur_act;
         c.act_next = sh.act[cur_act == sh.act[0]];
         c.queue_next = sh.queue[0];
+        c.sr = D.sr + 1;            // the sub-round its claims are for
         run(kFastRound, c, nact);
         cur_act = c.act_next;
         cur_q = sh.queue[0];
+        checked = true;
         nact = sh.n_next;
         nq = sh.n_queue;
         D.errs |= word(&c.cnt->err[c.eslot]);
@@ -290,6 +299,7 @@ __device__ __forceinline__ void fast_flips(SH& sh) {
     int nq = (int)sh.count, sub = 0, turn = 0, flips = 0;
     const int budget = sh.budget;
     int carried = sh.ctx.carry_n;               // leading entries carried over from the previous round
+    bool checked = sh.checked;
     if (tid == 0) { sh.tally[0][0] = 0; sh.tally[0][1] = 0; }
     fast_sync<SH::kCap>();
     do {
@@ -302,10 +312,15 @@ __device__ __forceinline__ void fast_flips(SH& sh) {
         int2 cd = make_int2(-1, -1);
         if (tid < nq) {
             qe = q[tid];
-            cd = flip_candidate(c, qe, tid < carried);
-            if (cd.x >= 0) claim_pair(c, cd);
+            if (checked) {
+                cd = sh.cand[tid];
+            } else {
+                cd = flip_candidate(c, qe, tid < carried);
+                if (cd.x >= 0) claim_pair(c, cd);
+            }
         }
-        fast_sync<SH::kCap>();
+        if (!checked) fast_sync<SH::kCap>();
+        checked = false;
         // flip
         const int t = cd.x >> 2, n = cd.y >> 2;
         FlipRows r;
@@ -380,10 +395,18 @@ __device__ __forceinline__ void fast_round(SH& sh) {
     fast_sync<SH::kCap>();
     if (code >= 0) {
         int4 qe;
-        const int n = fix_winner(c, make_int2(q * 8 + code, t), qe);
-        int* qn = sh.queue[0] + atomicAdd(&sh.n_queue, n);
+        int2 cd[4];
+        const int n = fix_winner<true>(c, make_int2(q * 8 + code, t), qe, cd);
+        const int at = atomicAdd(&sh.n_queue, n);
+        int* qn = sh.queue[0] + at;
         qn[0] = qe.x; qn[1] = qe.y; qn[2] = qe.z;
         if (n == 4) qn[3] = qe.w;
+        // the candidates are used if the queue is short enough for fast_flips
+        if (at + n <= SH::kCap) {
+            int2* cn = sh.cand + at;
+            cn[0] = cd[0]; cn[1] = cd[1]; cn[2] = cd[2];
+            if (n == 4) cn[3] = cd[3];
+        }
     }
 }
 
@@ -404,6 +427,8 @@ __device__ __forceinline__ Ctx items_view(const Ctx& p, int k) {
         if (k == K_FLIP_FIX) { c.list_n = p.list_n; c.base_q = p.base_q; }
     } else if (k == K_FIX) {
         c.winners = p.winners; c.queue_next = p.queue_next; c.base_q = p.base_q;
+        c.sr = p.sr; c.cand = p.cand; c.claim = p.claim; c.P = p.P;
+        __builtin_assume(__isGlobal(c.claim)); __builtin_assume(__isGlobal(c.P));
     } else {        // K_RELOC_VOTE, K_SPLIT
         c.act = p.act; c.loc = p.loc; c.pedge = p.pedge; c.vote = p.vote;
         __builtin_assume(__isGlobal(c.loc)); __builtin_assume(__isGlobal(c.pedge)); __builtin_assume(__isGlobal(c.vote));
@@ -422,6 +447,8 @@ __device__ __forceinline__ void round_items(const SH& sh) {
             const int ks[1] = {i};
             const int2 f[1] = {flip_first(c, FP_FIX, i)};
             flip_fix_multi_f<1>(c, ks, f);
+        } else if constexpr (K == K_FIX) {
+            fix_winner_queue<true>(c, c.winners[i]);
         } else {
             dispatch(K, c, i);
         }

@@ -712,14 +712,17 @@ GCDT_HD void body_split(const Ctx& c, int k) {
 // 2 in 2+2q', 3+2q'; an edge split leaves q' where m's one outer edge it
 // keeps faces and its other outer edge in 2+2q' (first triangle) or 3+2q'
 // (second triangle, bit 3 of the flags).
-GCDT_HD int split_child(const int4& cv, int s, const int4& mv, int m, int ms) {
+// *opp: the vertex opposite that edge, which is m's inserted point in every
+// child.
+GCDT_HD int split_child(const int4& cv, int s, const int4& mv, int m, int ms, int* opp) {
     const int u = comp(cv, nx3(s)), v = comp(cv, nx3(nx3(s)));
     const int p1 = nx3(ms), p2 = nx3(p1);
     const int w1 = comp(mv, p1), w2 = comp(mv, p2);
     const bool k1 = w1 == u || w1 == v, k2 = w2 == u || w2 == v;
-    if (k1 && k2) return m;
+    if (k1 && k2) { *opp = comp(mv, ms); return m; }
     const int p = k1 ? p2 : p1;
     const int qm = comp(mv, p);
+    *opp = qm;
     return 2 + 2 * qm + (ms == nx3(p) ? ((mv.w >> 3) & 1) : 1);
 }
 
@@ -730,79 +733,6 @@ GCDT_HD int qtri(int e) { return (int)((unsigned)e >> 3); }
 
 // The children of the inserted points are distinct triangles, so the first
 // flip queue of a round needs no de-duplication.
-
-// The old edges of a split's children, for one inserted point: the edge in
-// slot s of child ch names its old neighbour; point it at the neighbour's
-// child that holds the edge when the neighbour was split in this round too
-// (its adjacency row's round stamp; flips of the round come after this
-// phase), else write ch into the neighbour's row.  The neighbour's record is
-// the sector the second case writes anyway.  All loads come before the first
-// write (they read no word that this phase writes), so that the three or four
-// edges' chains run side by side instead of one after the other.
-template <int E>
-GCDT_HD void resolve_split_edges(const Ctx& c, const int (&ch)[E], const int (&s)[E]) {
-    int old[E];
-    int4 cv[E], mv[E];
-    int mr[E];
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        old[k] = ((const int*)&tri_a(c, ch[k]))[s[k]];
-        cv[k] = tri_v(c, ch[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        mv[k] = old[k] >= 0 ? tri_v(c, old[k] >> 2) : make_int4(0, 0, 0, 0);
-        mr[k] = old[k] >= 0 ? tri_a(c, old[k] >> 2).w : 0;
-    }
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        if (old[k] < 0) continue;
-        const int m = old[k] >> 2, ms = old[k] & 3;
-        if (mr[k] == (int)c.round) ((int*)&tri_a(c, ch[k]))[s[k]] = enc(split_child(cv[k], s[k], mv[k], m, ms), ms);
-        else ((int*)&tri_a(c, m))[ms] = enc(ch[k], s[k]);
-    }
-}
-
-// Resolve outer adjacency of the children of one inserted point (w: the
-// winner entry) and give the flip-queue entries of the children, qe[0..n-1];
-// returns n (3, or 4 on an edge).
-GCDT_HD int fix_winner(const Ctx& c, int2 w, int4& qe) {
-    int q = w.x >> 3, t = w.y;
-    int T1 = 2 + 2 * q, T2 = 3 + 2 * q;
-    int code = w.x & 7;
-    // Only the old edges need a test: a spoke from q to a corner of the split
-    // triangle is locally Delaunay (q lies inside the old empty circumcircle,
-    // so the circle through q and the spoke's far edge excludes the third
-    // corner; on an edge split the spoke's quadrilateral is not even convex).
-    if (code == 7) {
-        const int ch[3] = {t, T1, T2}, sl[3] = {0, 1, 2};
-        resolve_split_edges<3>(c, ch, sl);
-        qe = make_int4(qentry(t, 1), qentry(T1, 2), qentry(T2, 4), 0);
-        return 3;
-    }
-    int e = code;
-    int e1 = nx3(e), e_2 = nx3(e1);
-    int en = comp(tri_a(c, T1), e);     // A2 slot e = enc(B1, e2)
-    int n = en >> 2, e2 = en & 3;
-    int f1 = nx3(e2), f2 = nx3(f1);
-    const int ch[4] = {t, T1, n, T2}, sl[4] = {e1, e_2, f1, f2};
-    resolve_split_edges<4>(c, ch, sl);
-    // outer edge and the half of the split edge
-    qe = make_int4(qentry(t, (1 << e1) | (1 << e)), qentry(T1, (1 << e_2) | (1 << e)),
-                   qentry(n, (1 << f1) | (1 << e2)), qentry(T2, (1 << f2) | (1 << e2)));
-    return 4;
-}
-// The same, the entries queued for the flip phase.
-GCDT_HD void body_fix_f(const Ctx& c, int2 w) {
-    int4 qe;
-    const int n = fix_winner(c, w, qe);
-    int* qn = c.queue_next + append_slots(&c.cnt->cur_q, c.base_q, n);
-    qn[0] = qe.x; qn[1] = qe.y; qn[2] = qe.z;
-    if (n == 4) qn[3] = qe.w;
-}
-GCDT_HD void body_fix(const Ctx& c, int k) { body_fix_f(c, c.winners[k]); }
-
-// ---------------------------------------------------------------- flips
 
 GCDT_HD unsigned long long claim_key(const Ctx& c, int key) {
     return ((unsigned long long)c.sr << 32) | (0xffffffffu - hash32((uint32_t)key));
@@ -821,6 +751,140 @@ GCDT_HD int first_bad_edge(int live, int2 a, int2 b, int2 cc, int2 p0, int2 p1, 
     }
     return -1;
 }
+
+// Claim both triangles of a candidate edge.  The claim
+// priority hash32(4t+i) is unique (hash32 is a bijection); the smallest wins
+// both triangles (atomicMax of its complement), so conflicts resolve like a
+// random-priority independent set, whatever the schedule.
+GCDT_HD void claim_pair(const Ctx& c, int2 cd) {
+    const unsigned long long ck = claim_key(c, cd.x);
+    at_max64(&c.claim[cd.x >> 2], ck);
+    at_max64(&c.claim[cd.y >> 2], ck);
+}
+// The old edges of a split's children, for one inserted point: the edge in
+// slot s of child ch names its old neighbour; point it at the neighbour's
+// child that holds the edge when the neighbour was split in this round too
+// (its adjacency row's round stamp; flips of the round come after this
+// phase), else write ch into the neighbour's row.  The neighbour's record is
+// the sector the second case writes anyway.  All loads come before the first
+// write (they read no word that this phase writes), so that the three or four
+// edges' chains run side by side instead of one after the other.
+//
+// kCheck: the children's first flip check as well (flip_candidate of each
+// queue entry): the neighbour across a child's old edge and the vertex
+// opposite it are known here, whatever the neighbour's own fix still has to
+// write.  half[k]: the slot of the half of a split edge in child k (-1: split
+// inside), whose other side is child sib[k]'s half.  cd[k]: the candidate.
+template <int E, bool kCheck>
+GCDT_HD void resolve_split_edges(const Ctx& c, const int (&ch)[E], const int (&s)[E], const int (&half)[E],
+                                 const int (&sib)[E], int2* cd) {
+    int old[E];
+    int4 cv[E], mv[E];
+    int mr[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        old[k] = ((const int*)&tri_a(c, ch[k]))[s[k]];
+        cv[k] = tri_v(c, ch[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        mv[k] = old[k] >= 0 ? tri_v(c, old[k] >> 2) : make_int4(0, 0, 0, 0);
+        mr[k] = old[k] >= 0 ? tri_a(c, old[k] >> 2).w : 0;
+    }
+    int now[E], opp[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        now[k] = -1;
+        opp[k] = 0;
+        if (old[k] < 0) continue;
+        const int m = old[k] >> 2, ms = old[k] & 3;
+        if (mr[k] == (int)c.round) {
+            now[k] = enc(split_child(cv[k], s[k], mv[k], m, ms, &opp[k]), ms);
+            ((int*)&tri_a(c, ch[k]))[s[k]] = now[k];
+        } else {
+            now[k] = old[k];
+            opp[k] = comp(mv[k], ms);
+            ((int*)&tri_a(c, m))[ms] = enc(ch[k], s[k]);
+        }
+    }
+    if (!kCheck) return;
+    int2 po[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) po[k] = c.P[opp[k]];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        const int4 v = cv[k];
+        int live = (now[k] >= 0) << s[k];
+        int2 ph = make_int2(0, 0);
+        if (half[k] >= 0) {
+            live |= 1 << half[k];
+            int4 o = cv[0];
+#pragma unroll
+            for (int u = 1; u < E; ++u)
+                if (sib[k] == u) o = cv[u];
+            ph = c.P[comp(o, half[sib[k]])];
+        }
+        live &= ~v.w;
+        const int i = first_bad_edge(live, c.P[v.x], c.P[v.y], c.P[v.z], s[k] == 0 ? po[k] : ph,
+                                     s[k] == 1 ? po[k] : ph, s[k] == 2 ? po[k] : ph);
+        cd[k] = make_int2(-1, -1);
+        if (i < 0) continue;
+        cd[k] = make_int2(enc(ch[k], i), i == s[k] ? now[k] : enc(ch[sib[k]], half[sib[k]]));
+        claim_pair(c, cd[k]);
+    }
+}
+
+// Resolve outer adjacency of the children of one inserted point (w: the
+// winner entry) and give the flip-queue entries of the children, qe[0..n-1];
+// returns n (3, or 4 on an edge).  kCheck: with their candidates, cd[0..n-1].
+template <bool kCheck>
+GCDT_HD int fix_winner(const Ctx& c, int2 w, int4& qe, int2 (&cd)[4]) {
+    int q = w.x >> 3, t = w.y;
+    int T1 = 2 + 2 * q, T2 = 3 + 2 * q;
+    int code = w.x & 7;
+    // Only the old edges need a test: a spoke from q to a corner of the split
+    // triangle is locally Delaunay (q lies inside the old empty circumcircle,
+    // so the circle through q and the spoke's far edge excludes the third
+    // corner; on an edge split the spoke's quadrilateral is not even convex).
+    if (code == 7) {
+        const int ch[3] = {t, T1, T2}, sl[3] = {0, 1, 2}, none[3] = {-1, -1, -1}, sib[3] = {0, 0, 0};
+        resolve_split_edges<3, kCheck>(c, ch, sl, none, sib, cd);
+        qe = make_int4(qentry(t, 1), qentry(T1, 2), qentry(T2, 4), 0);
+        return 3;
+    }
+    int e = code;
+    int e1 = nx3(e), e_2 = nx3(e1);
+    int en = comp(tri_a(c, T1), e);     // A2 slot e = enc(B1, e2)
+    int n = en >> 2, e2 = en & 3;
+    int f1 = nx3(e2), f2 = nx3(f1);
+    // A1 = t and B2 = T2 share a half of the split edge, A2 = T1 and B1 = n
+    const int ch[4] = {t, T1, n, T2}, sl[4] = {e1, e_2, f1, f2}, half[4] = {e, e, e2, e2}, sib[4] = {3, 2, 1, 0};
+    resolve_split_edges<4, kCheck>(c, ch, sl, half, sib, cd);
+    // outer edge and the half of the split edge
+    qe = make_int4(qentry(t, (1 << e1) | (1 << e)), qentry(T1, (1 << e_2) | (1 << e)),
+                   qentry(n, (1 << f1) | (1 << e2)), qentry(T2, (1 << f2) | (1 << e2)));
+    return 4;
+}
+// The same, the entries queued for the flip phase (kCheck: checked).
+template <bool kCheck>
+GCDT_HD void fix_winner_queue(const Ctx& c, int2 w) {
+    int4 qe;
+    int2 cd[4];
+    const int n = fix_winner<kCheck>(c, w, qe, cd);
+    const int at = append_slots(&c.cnt->cur_q, c.base_q, n);
+    int* qn = c.queue_next + at;
+    qn[0] = qe.x; qn[1] = qe.y; qn[2] = qe.z;
+    if (n == 4) qn[3] = qe.w;
+    if (kCheck) {
+        int2* cn = c.cand + at;
+        cn[0] = cd[0]; cn[1] = cd[1]; cn[2] = cd[2];
+        if (n == 4) cn[3] = cd[3];
+    }
+}
+GCDT_HD void body_fix_f(const Ctx& c, int2 w) { fix_winner_queue<false>(c, w); }
+GCDT_HD void body_fix(const Ctx& c, int k) { body_fix_f(c, c.winners[k]); }
+
+// ---------------------------------------------------------------- flips
 
 // The first edge of queue entry qe's triangle that is not locally Delaunay
 // (perturbed incircle > 0, not a constraint): (4t+i, 4n+j) of its two sides,
@@ -845,15 +909,6 @@ GCDT_HD int2 flip_candidate(const Ctx& c, int qe, bool carried) {
     return i < 0 ? make_int2(-1, -1) : make_int2(enc(t, i), comp(ta, i));
 }
 
-// Queue entry k: claim both triangles of its candidate edge.  The claim
-// priority hash32(4t+i) is unique (hash32 is a bijection); the smallest wins
-// both triangles (atomicMax of its complement), so conflicts resolve like a
-// random-priority independent set, whatever the schedule.
-GCDT_HD void claim_pair(const Ctx& c, int2 cd) {
-    const unsigned long long ck = claim_key(c, cd.x);
-    at_max64(&c.claim[cd.x >> 2], ck);
-    at_max64(&c.claim[cd.y >> 2], ck);
-}
 GCDT_HD void body_flip_check(const Ctx& c, int k) {
     const int2 cd = flip_candidate(c, c.queue[k], k < c.carry_n);
     if (cd.x >= 0) claim_pair(c, cd);

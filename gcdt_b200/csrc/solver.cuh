@@ -195,23 +195,39 @@ struct FastItems { static constexpr int value = 0; };
 template <class EX>
 struct FastItems<EX, decltype((void)EX::kFastItems)> { static constexpr int value = EX::kFastItems; };
 
+// An executor with kFixChecks finds the flip candidates of the split's
+// children in the split fix (fix_winner), which has their neighbours at hand:
+// one block's short lists, where a phase more costs its latency (4,096
+// batched instances 64.8 -> 63.1 ms).  On the grid the first check is cheap
+// (a split's entries share their rows in L1: 0.7 of 3.7 ms of the headline's
+// checks) and the longer fix is not (1.05 -> 3.3 ms).
+template <class EX, class = void>
+struct FixChecks { static constexpr bool value = false; };
+template <class EX>
+struct FixChecks<EX, decltype((void)EX::kFixChecks)> { static constexpr bool value = EX::kFixChecks; };
+
 // Flip sub-rounds on the queue `D.qa` (nq entries, stamped D.sr) until it
 // has at most `stop` entries after at least one sub-round, or -- for the
 // single-block tail -- until it grows past max_nq.  The first sub-round
-// always runs, so an entry is carried over at most one round.
+// always runs, so an entry is carried over at most one round.  checked: the
+// entries after the carried ones have their candidates already.  (The
+// single-block tails check them again: the same candidates and claims.)
 template <class EX>
-GCDT_HD int flip_loop(EX& ex, Ctx& c, Driver& D, long long& nq, long long max_nq, long long stop = 0) {
+GCDT_HD int flip_loop(EX& ex, Ctx& c, Driver& D, long long& nq, long long max_nq, long long stop = 0,
+                      bool checked = false) {
     long long guard = 0;
     const long long budget = budget_subrounds(c);
     while (nq > 0 && nq <= max_nq && (guard == 0 || nq > stop)) {
         if (++guard > budget) return ST_ITER_LIMIT;
         if (EX::kCanNarrow && nq <= c.narrow_q) {
+            checked = false;
             int rc = ex.narrow_flips(c, D, nq);
             if (rc || D.errs) return rc ? rc : D.errs;
             continue;
         }
         if constexpr (FastItems<EX>::value > 0) {
             if (nq <= FastItems<EX>::value && nq <= max_nq && stop == 0) {
+                checked = false;
                 long long left = budget - guard + 1;
                 const int rc = ex.fast_flips(c, D, nq, left);
                 if (rc) return rc;
@@ -223,8 +239,10 @@ GCDT_HD int flip_loop(EX& ex, Ctx& c, Driver& D, long long& nq, long long max_nq
         c.base_q = D.e_q;
         c.base_flip = D.e_flip;
         c.carry_n = (int)D.drop;
+        const long long unchecked = checked ? D.drop : nq;
+        checked = false;
         D.drop = 0;
-        run_phase(ex, c, D, K_FLIP_CHECK, nq);
+        if (unchecked > 0) run_phase(ex, c, D, K_FLIP_CHECK, unchecked);
         run_phase(ex, c, D, K_FLIP_DO, nq);
         D.e_flip = ex.cursor(&c.cnt->cur_flip);
         if (D.errs) return D.errs;
@@ -308,7 +326,7 @@ GCDT_HD int insert_rounds(EX& ex, Ctx& c, Driver& D, long long nact, bool voted 
         long long nq = (long long)(D.e_q - c.base_q);
         D.drop = D.carry;
         D.carry = 0;
-        int rc = flip_loop(ex, c, D, nq, (long long)1 << 62, EX::kCanNarrow ? (long long)c.carry_q : 0);
+        int rc = flip_loop(ex, c, D, nq, (long long)1 << 62, EX::kCanNarrow ? (long long)c.carry_q : 0, FixChecks<EX>::value);
         if (rc) return rc;
         D.carry = nq;
     }
