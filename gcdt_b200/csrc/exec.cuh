@@ -272,7 +272,8 @@ struct BlockExecT {
 // level; their phases are a few hundred dependent instructions on a few
 // warps, so publishing each phase, its lists in memory and generic
 // addressing cost more than its work (a flip sub-round of the tails 5.6 ->
-// 2.2 us: check 1.1, flip 0.45, fix 0.65; a round's insertion 9 -> 4.8 us).
+// 2.2 us, 1.8 with fix and check in one phase; a round's insertion 9 -> 4.8
+// us).
 
 constexpr int kBarFast = 3;
 template <int CAP>
@@ -290,80 +291,78 @@ __device__ __forceinline__ Ctx fast_view(const Ctx& p) {
     return c;
 }
 
+// Sub-rounds of two phases each: the fix of one and the check of the next are
+// one (fix_and_check).  Between them the queue holds the flipped triangles
+// from its front and the losers, those flipped by others among them, from
+// its end.
 template <class SH>
 __device__ __forceinline__ void fast_flips(SH& sh) {
+    constexpr int kEnd = 4 * SH::kCap - 1;
     Ctx c = fast_view(sh.ctx);
     const int tid = threadIdx.x;
     const int* q = sh.ctx.queue;
     int buf = sh.ctx.queue == sh.queue[0];      // the buffer the next queue goes to
-    int nq = (int)sh.count, sub = 0, turn = 0, flips = 0;
+    int nq = (int)sh.count, nfix = 0, sub = 0, turn = 0, flips = 0;
     const int budget = sh.budget;
-    int carried = sh.ctx.carry_n;               // leading entries carried over from the previous round
-    bool checked = sh.checked;
     if (tid == 0) { sh.tally[0][0] = 0; sh.tally[0][1] = 0; }
-    fast_sync<SH::kCap>();
-    do {
+    // the first check, of a queue without flips to fix
+    int qe = 0;
+    int2 cd = make_int2(-1, -1);
+    if (tid < nq) {
+        qe = q[tid];
+        if (sh.checked) {
+            cd = sh.cand[tid];
+        } else {
+            cd = flip_candidate(c, qe, tid < sh.ctx.carry_n);   // leading entries carried over from the previous round
+            if (cd.x >= 0) claim_pair(c, cd);
+        }
+    }
+    int* qn;
+    for (;;) {
+        fast_sync<SH::kCap>();
+        // flip
         int* tally = sh.tally[turn];
-        int* qn = sh.queue[buf];
+        qn = sh.queue[buf];
         turn = turn == 2 ? 0 : turn + 1;
         if (tid == 0) { sh.tally[turn][0] = 0; sh.tally[turn][1] = 0; }
-        // check
-        int qe = 0;
-        int2 cd = make_int2(-1, -1);
-        if (tid < nq) {
-            qe = q[tid];
-            if (checked) {
-                cd = sh.cand[tid];
-            } else {
-                cd = flip_candidate(c, qe, tid < carried);
-                if (cd.x >= 0) claim_pair(c, cd);
-            }
-        }
-        if (!checked) fast_sync<SH::kCap>();
-        checked = false;
-        // flip
-        const int t = cd.x >> 2, n = cd.y >> 2;
-        FlipRows r;
-        bool won = false;
         if (cd.x >= 0) {
+            const int t = cd.x >> 2, n = cd.y >> 2;
             const unsigned long long ck = claim_key(c, cd.x);
             const unsigned long long c0 = ld_l2(&c.claim[t]), c1 = ld_l2(&c.claim[n]);
-            won = c0 == ck && c1 == ck;
-            if (won) {
-                r = do_flip(c, t, cd.x & 3, n, cd.y & 3, tri_v(c, t), tri_a(c, t), tri_v(c, n), tri_a(c, n));
+            if (c0 == ck && c1 == ck) {
+                do_flip(c, t, cd.x & 3, n, cd.y & 3, tri_v(c, t), tri_a(c, t), tri_v(c, n), tri_a(c, n));
                 int* qp = qn + 2 * atomicAdd(&tally[0], 1);
                 qp[0] = qentry(t, 5);
                 qp[1] = qentry(n, 3);
+            } else {
+                qn[kEnd - atomicAdd(&tally[1], 1)] = qe;
             }
         }
         fast_sync<SH::kCap>();
-        // fix: the flip's outer edges; a loser that nobody flipped goes back
-        const int nflip = tally[0];
-        if (won) {
-            const int4 none = make_int4(-1, -1, -1, -1);
-            const int2 nil = make_int2(-1, -1);
-            const int o0 = r.ta.x, o2 = r.ta.z, u0 = r.na.x, u1 = r.na.y;     // old outer neighbours
-            const int4 m0 = o0 >= 0 ? tri_v(c, o0 >> 2) : none, m2 = o2 >= 0 ? tri_v(c, o2 >> 2) : none;
-            const int4 g0 = u0 >= 0 ? tri_v(c, u0 >> 2) : none, g1 = u1 >= 0 ? tri_v(c, u1 >> 2) : none;
-            const int2 p0 = o0 >= 0 ? partner_slots(c, o0 >> 2) : nil, p2 = o2 >= 0 ? partner_slots(c, o2 >> 2) : nil;
-            const int2 q0 = u0 >= 0 ? partner_slots(c, u0 >> 2) : nil, q1 = u1 >= 0 ? partner_slots(c, u1 >> 2) : nil;
-            resolve_flip_loaded(c, t, r.tv, 0, o0, m0, p0);
-            resolve_flip_loaded(c, t, r.tv, 2, o2, m2, p2);
-            resolve_flip_loaded(c, n, r.nv, 0, u0, g0, q0);
-            resolve_flip_loaded(c, n, r.nv, 1, u1, g1, q1);
-        } else if (cd.x >= 0 && flip_stamp(tri_v(c, t).w) != (int)c.sr) {
-            qn[2 * nflip + atomicAdd(&tally[1], 1)] = qe;
-        }
-        fast_sync<SH::kCap>();
-        nq = 2 * nflip + tally[1];
-        flips += nflip;
+        nfix = 2 * tally[0];
+        nq = nfix + tally[1];
+        flips += tally[0];
         c.sr++;
         ++sub;
-        carried = 0;
         q = qn;
         buf ^= 1;
-    } while (nq > 0 && nq <= SH::kCap && sub < budget);
-    if (tid == 0) { sh.n_queue = nq; sh.subrounds = sub; sh.flips = flips; }
+        if (nq == 0 || nq > SH::kCap || sub >= budget) break;
+        // fix and check
+        cd = make_int2(-1, -1);
+        if (tid < nq) {
+            qe = q[tid < nfix ? tid : kEnd - (tid - nfix)];
+            cd = fix_and_check(c, qe, tid < nfix);
+        }
+    }
+    // leave a queue as the phases do: fixed, the losers that nobody flipped
+    // after the flipped triangles (at most 3 CAP entries in all: the raw
+    // losers are beyond them)
+    for (int i = tid; i < nq; i += SH::kCap) {
+        const int e = q[i < nfix ? i : kEnd - (i - nfix)];
+        if (fix_entry(c, e, i < nfix) && i >= nfix) qn[nfix + atomicAdd(&sh.tally[turn][0], 1)] = e;
+    }
+    fast_sync<SH::kCap>();
+    if (tid == 0) { sh.n_queue = nfix + sh.tally[turn][0]; sh.subrounds = sub; sh.flips = flips; }
 }
 
 template <class SH>

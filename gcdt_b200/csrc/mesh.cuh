@@ -1034,8 +1034,8 @@ GCDT_HD FlipRows do_flip(const Ctx& c, int t, int i, int n, int j,
 // DC, CA, so the partner's slot follows from whether the edge ends at D.
 // Otherwise -1 (the old neighbour keeps the edge).  The partner slots are
 // the flip's new diagonal, which no fix pass writes.
-GCDT_HD int moved_edge(const Ctx& c, const int4& tv, int s, int old, const int4& mv, int2 mp) {
-    if (flip_stamp(mv.w) != (int)c.sr) return -1;
+GCDT_HD int moved_edge(int sr, const int4& tv, int s, int old, const int4& mv, int2 mp) {
+    if (flip_stamp(mv.w) != sr) return -1;
     const int u = comp(tv, nx3(s)), v = comp(tv, nx3(nx3(s)));
     const int su = slot_of_or_none(mv, u), sv = slot_of_or_none(mv, v);
     if (su >= 0 && sv >= 0) return enc(old >> 2, 3 - su - sv);
@@ -1118,7 +1118,7 @@ GCDT_HD void resolve_flip_edge(const Ctx& c, int tt, int s) {
     int old = comp(*row, s);
     if (old < 0) return;
     int m = old >> 2, ms = old & 3;
-    const int e = moved_edge(c, tri_v(c, tt), s, old, tri_v(c, m), partner_slots(c, m));
+    const int e = moved_edge((int)c.sr, tri_v(c, tt), s, old, tri_v(c, m), partner_slots(c, m));
     if (e >= 0) ((int*)row)[s] = e;
     else ((int*)&tri_a(c, m))[ms] = enc(tt, s);
 }
@@ -1147,7 +1147,7 @@ GCDT_HD void body_flip_fix(const Ctx& c, int k) {
 // resolve_flip_edge would make.
 GCDT_HD void resolve_flip_loaded(const Ctx& c, int tt, const int4& tv, int s, int old, const int4& mv, int2 mp) {
     if (old < 0) return;
-    const int e = moved_edge(c, tv, s, old, mv, mp);
+    const int e = moved_edge((int)c.sr, tv, s, old, mv, mp);
     if (e >= 0) ((int*)&tri_a(c, tt))[s] = e;
     else ((int*)&tri_a(c, old >> 2))[old & 3] = enc(tt, s);
 }
@@ -1228,6 +1228,63 @@ GCDT_HD void body_flip_fix_pair(const Ctx& c, int k0, int k1) {
     const int ks[2] = {k0, k1};
     const int2 f[2] = {flip_first(c, FP_FIX, k0), flip_first(c, FP_FIX, k1)};
     flip_fix_multi_f<2>(c, ks, f);
+}
+
+// The flip fix of sub-round c.sr - 1 and the check of c.sr in one, for one
+// entry of a queue that holds the previous sub-round's flipped triangles
+// (flipped: their edges in the mask are their outer ones, to be resolved) and
+// its losers, flipped by another thread or not.  Which triangle holds an
+// edge now follows from rows that no fix writes (moved_edge), so the check
+// need not wait for the other threads' fixes; a slot that one of them has
+// rewritten already gives the same answer.  Claims the candidate and returns
+// it, or (-1, -1).
+GCDT_HD int2 fix_and_check(const Ctx& c, int qe, bool flipped) {
+    const int t = qtri(qe), mask = qe & 7, prev = (int)c.sr - 1;
+    const int4 tv = tri_v(c, t), ta = tri_a(c, t);
+    if (!flipped && flip_stamp(tv.w) == prev) return make_int2(-1, -1);
+    int old[3], now[3], d[3];
+    int4 mv[3];
+    int2 mp[3];
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        old[s] = (mask >> s) & 1 ? comp(ta, s) : -1;
+        mv[s] = old[s] >= 0 ? tri_v(c, old[s] >> 2) : make_int4(0, 0, 0, 0);
+        mp[s] = old[s] >= 0 ? partner_slots(c, old[s] >> 2) : make_int2(0, 0);
+    }
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        now[s] = -1;
+        d[s] = 0;
+        if (old[s] < 0) continue;
+        const int e = moved_edge(prev, tv, s, old[s], mv[s], mp[s]);
+        now[s] = e >= 0 ? e : old[s];
+        d[s] = (now[s] >> 2) == (old[s] >> 2) ? comp(mv[s], now[s] & 3) : comp(tri_v(c, now[s] >> 2), now[s] & 3);
+        if (!flipped) continue;
+        if (e >= 0) ((int*)&tri_a(c, t))[s] = e;
+        else ((int*)&tri_a(c, old[s] >> 2))[old[s] & 3] = enc(t, s);
+    }
+    const int live = ((now[0] >= 0) | ((now[1] >= 0) << 1) | ((now[2] >= 0) << 2)) & ~tv.w;
+    const int i = first_bad_edge(live, c.P[tv.x], c.P[tv.y], c.P[tv.z], c.P[d[0]], c.P[d[1]], c.P[d[2]]);
+    if (i < 0) return make_int2(-1, -1);
+    const int2 cd = make_int2(enc(t, i), i == 0 ? now[0] : (i == 1 ? now[1] : now[2]));
+    claim_pair(c, cd);
+    return cd;
+}
+
+// The fix of that entry alone; false for a loser that was flipped (no entry
+// of the queue any more).
+GCDT_HD bool fix_entry(const Ctx& c, int qe, bool flipped) {
+    const int t = qtri(qe), prev = (int)c.sr - 1;
+    if (!flipped) return flip_stamp(tri_v(c, t).w) != prev;
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        const int old = (qe >> s) & 1 ? comp(tri_a(c, t), s) : -1;
+        if (old < 0) continue;
+        const int e = moved_edge(prev, tri_v(c, t), s, old, tri_v(c, old >> 2), partner_slots(c, old >> 2));
+        if (e >= 0) ((int*)&tri_a(c, t))[s] = e;
+        else ((int*)&tri_a(c, old >> 2))[old & 3] = enc(t, s);
+    }
+    return true;
 }
 
 // ---------------------------------------------------------------- constraints
