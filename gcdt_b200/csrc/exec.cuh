@@ -380,7 +380,7 @@ __device__ __forceinline__ void fast_round(SH& sh) {
     int code = -1;
     if (t >= 0) {
         const unsigned long long key = vote_key(c, q);
-        if (ld_l2(&c.vote[t]) == key) code = split_rows(c, q, t, e, key);
+        if (ld_l2(&c.vote[t]) == key && won_across(c, t, e, key)) code = split_rows(c, q, t, e);
     }
     // survivors, by warp
     const unsigned alive = __ballot_sync(0xffffffffu, t >= 0), next = __ballot_sync(0xffffffffu, t >= 0 && code < 0);

@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(kBlock) gcdt_activate(Ctx c, int level) {
     c.base_act = c.cnt->handoff[offsetof(Driver, e_act0) / 8];
     c.round = reinterpret_cast<const unsigned*>(c.cnt->handoff)[offsetof(Driver, round) / 4] + 1;
     if (c.lvl[i] != level) return;
+    c.act_next[append_slot(&c.cnt->cur_act0, c.base_act)] = i;
     const int2 p = c.P[i];
     const int t = activate_location(c, i, p);
     if (t < 0) { fail(c, ST_ITER_LIMIT); return; }
@@ -173,7 +174,6 @@ __global__ void __launch_bounds__(kBlock) gcdt_activate(Ctx c, int level) {
     const int e = edge_of(c, t, p);
     c.loc[i] = t;
     c.pedge[i] = (signed char)e;
-    c.act_next[append_slot(&c.cnt->cur_act0, c.base_act)] = i;
     cast_votes(c, i, t, e);
 }
 __global__ void __launch_bounds__(kBlock) gcdt_output(Ctx c) {

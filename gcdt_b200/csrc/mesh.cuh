@@ -519,10 +519,10 @@ GCDT_HD int activate_location(const Ctx& c, int i, int2 p) {
 }
 GCDT_HD void body_activate(const Ctx& c, int i) {
     if (c.lvl[i] != c.level) return;
+    c.act_next[append_slot(&c.cnt->cur_act0, c.base_act)] = i;      // before the walk, as in the relocation
     const int t = activate_location(c, i, c.P[i]);
     if (t < 0) { fail(c, ST_ITER_LIMIT); return; }
     c.loc[i] = t;
-    c.act_next[append_slot(&c.cnt->cur_act0, c.base_act)] = i;
 }
 
 GCDT_HD int at_min(int* p, int v) {
@@ -622,10 +622,12 @@ GCDT_HD void cast_votes(const Ctx& c, int q, int t, int e) {
 // caller): relocate, keep it in the next list, and vote.
 GCDT_HD void body_reloc_vote_qt(const Ctx& c, int q, int t, int2 p) {
     if (t < 0) return;                       // inserted last round
+    // the list first, while the warp is together: after the walks it takes an
+    // atomic per group of lanes that happen to end together
+    c.act_next[append_slot(&c.cnt->cur_act, c.base_act)] = q;
     int e;
     t = relocate(c, q, t, p, &e);
     if (t < 0) return;
-    c.act_next[append_slot(&c.cnt->cur_act, c.base_act)] = q;
     c.pedge[q] = (signed char)e;
     cast_votes(c, q, t, e);
 }
@@ -637,9 +639,14 @@ GCDT_HD void body_reloc_vote(const Ctx& c, int k) {
 // Winners split their triangle(s).  Child j of a split triangle is the
 // triangle with vertex j replaced by q; it keeps the old edge j in slot j.
 // Outer adjacency is written as the old neighbour and resolved in body_fix.
-// Returns the winner's split code (7: inside, else the split edge's slot),
-// or -1 if q lost the triangle across the edge it lies on.
-GCDT_HD int split_rows(const Ctx& c, int q, int t, int e, unsigned long long key) {
+// Whether point q on the edge in slot e of triangle t, which it won, won the
+// triangle across it too (e < 0: inside t).
+GCDT_HD bool won_across(const Ctx& c, int t, int e, unsigned long long key) {
+    return e < 0 || ld_l2(&c.vote[comp(tri_a(c, t), e) >> 2]) == key;
+}
+
+// Returns the split code (7: inside, else the split edge's slot).
+GCDT_HD int split_rows(const Ctx& c, int q, int t, int e) {
     int T1 = 2 + 2 * q, T2 = 3 + 2 * q;
     int4 tv = tri_v(c, t), ta = tri_a(c, t);
     int fl = tv.w;
@@ -659,7 +666,6 @@ GCDT_HD int split_rows(const Ctx& c, int q, int t, int e, unsigned long long key
     } else {
         int en = comp(ta, e);
         int n = en >> 2, e2 = en & 3;
-        if (ld_l2(&c.vote[n]) != key) return -1;
         int4 nv = tri_v(c, n), na = tri_a(c, n);
         int gl = nv.w;
         // children: A1 = child_{e+1}(t) -> t, A2 = child_{e+2}(t) -> T1,
@@ -695,8 +701,10 @@ GCDT_HD int split_rows(const Ctx& c, int q, int t, int e, unsigned long long key
 GCDT_HD void body_split_qt(const Ctx& c, int q, int t) {
     const unsigned long long key = vote_key(c, q);
     if (c.vote[t] != key) return;
-    const int code = split_rows(c, q, t, c.pedge[q], key);
-    if (code >= 0) c.winners[append_slot(&c.cnt->cur_win, c.base_win)] = make_int2(q * 8 + code, t);
+    const int e = c.pedge[q];
+    if (!won_across(c, t, e, key)) return;
+    int2* w = c.winners + append_slot(&c.cnt->cur_win, c.base_win);     // (while the warp is together)
+    *w = make_int2(q * 8 + split_rows(c, q, t, e), t);
 }
 GCDT_HD void body_split(const Ctx& c, int k) {
     const int q = c.act[k];
@@ -868,10 +876,11 @@ GCDT_HD int fix_winner(const Ctx& c, int2 w, int4& qe, int2 (&cd)[4]) {
 // The same, the entries queued for the flip phase (kCheck: checked).
 template <bool kCheck>
 GCDT_HD void fix_winner_queue(const Ctx& c, int2 w) {
+    const int n = (w.x & 7) == 7 ? 3 : 4;
+    const int at = append_slots(&c.cnt->cur_q, c.base_q, n);            // (while the warp is together)
     int4 qe;
     int2 cd[4];
-    const int n = fix_winner<kCheck>(c, w, qe, cd);
-    const int at = append_slots(&c.cnt->cur_q, c.base_q, n);
+    fix_winner<kCheck>(c, w, qe, cd);
     int* qn = c.queue_next + at;
     qn[0] = qe.x; qn[1] = qe.y; qn[2] = qe.z;
     if (n == 4) qn[3] = qe.w;
