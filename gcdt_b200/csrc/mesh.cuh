@@ -1543,9 +1543,10 @@ GCDT_HD void body_cproc(const Ctx& c, int k) {
 
 GCDT_HD void body_output(const Ctx& c, int t) {
     int4 tv = tri_v(c, t), ta = tri_a(c, t);
-    c.out_tris[3 * t + 0] = c.perm[tv.x];
-    c.out_tris[3 * t + 1] = c.perm[tv.y];
-    c.out_tris[3 * t + 2] = c.perm[tv.z];
+    const int a = c.perm[tv.x], b = c.perm[tv.y], d = c.perm[tv.z];     // before the first store
+    c.out_tris[3 * t + 0] = a;
+    c.out_tris[3 * t + 1] = b;
+    c.out_tris[3 * t + 2] = d;
     c.out_adj[3 * t + 0] = ta.x < 0 ? -1 : ta.x >> 2;
     c.out_adj[3 * t + 1] = ta.y < 0 ? -1 : ta.y >> 2;
     c.out_adj[3 * t + 2] = ta.z < 0 ? -1 : ta.z >> 2;
