@@ -47,11 +47,12 @@ sys.path.insert(0, ROOT)
 METRIC = "CDT Mpts/s at 10M pts+200k segs"
 UNIT = "Mpts/s"
 WORKLOAD = "plain CDT at scale: 10M Gaussian-mixture/uniform int32 points in [1,2^30-2]^2 + 3,125 star polygons (200,000 segments)"
-# DRAM bytes (read + write) of the stage kernel per point, from an ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum) of the same workload shape at
-# 1,020,608 points: 799,542,272 + 648,609,536 bytes.  Reported per solve as
-# this figure times N (the full-size capture would replay a 2.4 GB arena ~40x).
-DRAM_BYTES_PER_POINT = (799542272 + 648609536) / 1020608
+# DRAM bytes (read + write) of a solve's own kernels per point, from an ncu
+# capture (dram__bytes_read.sum + dram__bytes_write.sum over its launches) of
+# the same workload shape at 1,020,608 points: 979,018,240 + 516,101,888
+# bytes.  Reported per solve as this figure times N (a full-size capture would
+# replay a 2.4 GB arena).
+DRAM_BYTES_PER_POINT = (979018240 + 516101888) / 1020608
 
 
 def rank_info():
@@ -446,7 +447,8 @@ def run_ours(args):
                          "traffic": args.traffic if args.traffic is not None else DRAM_BYTES_PER_POINT * n,
                          "traffic_source": "given" if args.traffic is not None else
                                            "ncu DRAM bytes/point at 1.02M points x N",
-                         "kernel": "gcdt::gcdt_stages (persistent stage kernel, one launch per solve)",
+                         "kernel": "gcdt::gcdt_stages (persistent stage kernel, one launch per level, "
+                                   "with the maps, activations and output between)",
                          "kernel_ms": stage_med,
                          "unit_of_work": "one full solve; algorithmic bytes 8N+8S+25(2N+2) = %d" % b_alg,
                          "step_achieved": b_alg / (ms_local * 1e-3) / 1e9,

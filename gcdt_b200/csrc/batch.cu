@@ -4,13 +4,15 @@
 // point set per process).  Here one call triangulates thousands of
 // independent instances of uneven size:
 //   1. one kernel computes the Hilbert key of every point of every instance;
-//   2. one segmented radix sort orders each instance's points;
-//   3. one kernel with one block per instance runs the whole solve of that
-//      instance -- set-up, insertion rounds, flip sub-rounds, constraint
-//      rounds, output -- with the same stage driver as the single solve,
-//      phases separated by block barriers.  Blocks are issued largest
-//      instance first, so the hardware block scheduler acts as the
-//      per-instance work queue and balances the tail.
+//   2. one segmented radix sort, or two sorts of the whole batch, order each
+//      instance's points;
+//   3. one block per instance, or a cluster of two, four or eight for an
+//      instance that would outlast the rest of the batch, runs the whole
+//      solve of that instance -- set-up, insertion rounds, flip sub-rounds,
+//      constraint rounds, output -- with the same stage driver as the single
+//      solve.  Blocks are issued largest instance first, so the hardware
+//      block scheduler acts as the per-instance work queue and balances the
+//      tail.
 // Every instance works in its own slice of one arena laid out on the host.
 // Outputs are the single solve's, instance by instance: instance i's 2n_i+2
 // triangles start at triangle 2*P_i + 2*i (P_i = its first point), with

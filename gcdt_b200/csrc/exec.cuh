@@ -641,7 +641,7 @@ struct TeamExec {
     Counters* cnt;
     unsigned rank, size;                     // of the block in its team, of the team
     SH* sh;
-    unsigned spin_limit = 1u << 25;          // polls before a grid barrier wait gives up
+    unsigned spin_limit = 1u << 26;          // polls before a grid barrier wait gives up
     bool prof = false;                       // record the phase profile and balance (a launch constant)
     // Snapshot of the head of Counters (status, error words, list cursors),
     // word k in lane k, read right after each barrier.
@@ -669,7 +669,7 @@ struct TeamExec {
     // the barrier's parity, which its driver counts along.  One atomic per
     // block, whose result nobody waits for, and no reset.  The counter starts
     // each solve at 0 (it clears its counters).  Every wait is
-    // bounded: after spin_limit polls (2^25, about ten seconds, in a solve)
+    // bounded: after spin_limit polls (2^26, about twenty seconds, in a solve)
     // the block records ST_BARRIER and stops waiting, and once that bit is
     // set no block waits or works any more, so the kernel always ends.  A
     // poll is one L2 round trip and nothing else: sleeping 64 ns between

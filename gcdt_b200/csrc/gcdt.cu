@@ -93,12 +93,6 @@ __global__ void __launch_bounds__(kBlock) gcdt_rank_check(Ctx c) {
     body_seg_level0(c, k);
 }
 
-// The whole set-up of a small problem in one block: its launches took longer
-// than their work (eleven launches and a 60-bit device sort of eight passes,
-// 140 us at 4,000 points and 60 at 250; this kernel FILL and FILL).  The sort
-// is a bitonic network over (key, index) pairs in shared memory; its steps
-// of stride up to 32 stay inside a warp's 64 entries and need no block
-// barrier.
 __global__ void gcdt_predicates(const int2* q, int n, int* out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;

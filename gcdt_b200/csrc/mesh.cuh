@@ -90,9 +90,10 @@ struct Counters {
     unsigned long long wcur_sum[2];
 };
 
-// The persistent kernel's phases see the launch's context with the fields
-// the stage driver changes between phases copied in (phase_view in
-// exec.cuh): a field the driver starts to change goes into that list.
+// The phases' items see the launch's context with the fields the stage driver
+// changes between phases copied in (publish and phase_view, items_view and
+// fast_view in exec.cuh): a field the driver starts to change goes into those
+// lists.
 struct Ctx {
     int n;          // input points
     int s;          // input segments

@@ -138,12 +138,12 @@ GCDT_HD unsigned budget_crounds(const Ctx& c) {
                                                                               : kMaxConstraintRounds;
 }
 
-// The stage driver runs the same control flow on every GPU thread of the
-// persistent kernel (EX = grid executor: a phase is a grid-stride loop
-// followed by a grid barrier) and on the host for the CPU emulation
-// (EX = sequential executor).  Every value the driver branches on is read
-// right after a barrier and cannot change before the next barrier, so all
-// threads take the same branches:
+// The stage driver runs the same control flow in the driver warp of every
+// block of a team (EX = team executor: a phase is a loop over the team's
+// workers followed by a team barrier) or of one block (EX = block executor),
+// and on the host for the CPU emulation (EX = sequential executor).  Every
+// value the driver branches on is read right after a barrier and cannot
+// change before the next barrier, so all of them take the same branches:
 //   - a list cursor is read right after the phase that appended to it, and
 //     the phase after that never appends to the same cursor;
 //   - errors of phase k go to err[k & 1], read after phase k's barrier
@@ -152,7 +152,8 @@ GCDT_HD unsigned budget_crounds(const Ctx& c) {
 // EX provides: phase(kernel, ctx, count), cursor(u64*) -> u64,
 // word(int*) -> int, finish(...), and kCanNarrow: whether small flip queues
 // and small insertion tails can be handed to one block (narrow_flips,
-// narrow_rounds), which runs this same driver with block barriers.
+// narrow_rounds), which runs this same driver with block barriers; and, where
+// it has them, kFastItems and kFixChecks (below).
 
 struct Driver {
     int* actA; int* actB; int* qa; int* qb;
@@ -430,8 +431,8 @@ GCDT_HD int run_stages(EX& ex, Ctx c, int part = -1) {
 }
 
 // Host part: clear the per-solve arrays, key sort, gather, levels and
-// segment set-up, then hand over to the stages (one persistent kernel on the
-// GPU).  Everything is enqueued on the backend's stream without waiting:
+// segment set-up, then hand over to the stages (on the GPU the persistent
+// kernel, in parts for large solves).  Everything is enqueued on the backend's stream without waiting:
 // errors found by the set-up kernels make the stage kernel stop at once.
 // A backend with a prelude of its own (fewer, fused launches) does all of it
 // but the stages.

@@ -64,7 +64,8 @@ typedef struct {
     int64_t host_syncs;
     int64_t kernel_launches;
     double device_ms;          /* CUDA-event time of the whole solve */
-    double stage_ms;           /* CUDA-event time of the persistent stage kernel alone */
+    double stage_ms;           /* CUDA-event time of the stages: the persistent kernel or, from
+                                  200,000 points on, its parts and the launches between them */
 } gcdt_stats;
 
 /* Largest point count a context accepts (triangle ids must fit 29 bits). */
@@ -143,9 +144,9 @@ typedef struct {
     int32_t narrow_active;
 } gcdt_tuning;
 gcdt_status gcdt_set_tuning(gcdt_context* ctx, const gcdt_tuning* tuning);   /* NULL: the defaults */
-/* Blocks of the persistent stage kernel's launch for ctx's solves (0, the
-   default: every co-resident block, one per SM; larger values are capped
-   there).  Fewer blocks leave SMs to other work, so several contexts can
+/* Blocks of the persistent stage kernel's launches for ctx's solves (0, the
+   default: every co-resident block, one per SM, and eight for up to 15,000
+   points; larger values are capped there).  Fewer blocks leave SMs to other work, so several contexts can
    solve at once; the result does not depend on it.  No counterpart in the
    reference. */
 gcdt_status gcdt_set_grid_blocks(gcdt_context* ctx, int32_t blocks);
@@ -180,8 +181,9 @@ gcdt_status gcdt_time_barriers(int device, int32_t rounds, double* us_per_barrie
 /* Per-phase profiling of ctx's later solves (no counterpart in the
    reference): on (nonzero), the stage kernel records the two read-outs
    below; off (the default), it records neither and their counters stay 0.
-   The records cost a few atomics and counter updates per phase (0.5% of
-   the 10M-point solve), so timed runs leave it off.  Returns GCDT_OK, or
+   The records cost a few atomics and counter updates per phase, and a
+   profiled solve runs all phases in the one kernel (6% more on the 10M-point
+   solve), so timed runs leave it off.  Returns GCDT_OK, or
    GCDT_BAD_INPUT for a null ctx. */
 gcdt_status gcdt_set_profiling(gcdt_context* ctx, int32_t on);
 
