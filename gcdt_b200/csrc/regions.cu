@@ -152,6 +152,11 @@ __global__ void __launch_bounds__(kBlock) k_seed(const int* adj, const int* list
         if (list[i] < 0) body_seed(adj, list[i] & INT_MAX, parent, level);
 }
 
+__global__ void __launch_bounds__(kBlock) k_seed_all(const int* adj, int nt, const int* parent, int* level) {
+    const int t = blockIdx.x * kBlock + threadIdx.x;
+    if (t < nt) body_seed(adj, t, parent, level);
+}
+
 // Few triangles have a constraint edge, so a pass is one read of the flags:
 // several triangles per thread keep their loads in flight together.
 constexpr int kExpandItems = 8;
@@ -182,7 +187,9 @@ using namespace gcdt_regions;
 // Scratch: flags (error word, list length, one change word per round
 // parity), the parent array and the per-root level array.  The list of
 // triangles that the tiles hand to the global passes is kept in d_depth,
-// which the last pass writes.
+// which the last pass writes; or, for a caller whose d_depth lies over the
+// inputs, in the level array, whose own use begins after the join (the box
+// triangles are then found by another read of the adjacency).
 extern "C" size_t gcdt_classify_regions_scratch_bytes(int32_t n_tris) {
     if (n_tris < 0 || n_tris > INT_MAX / 3) return 0;
     return 256 + 2 * align256(4 * (size_t)n_tris);
@@ -204,16 +211,24 @@ extern "C" gcdt_status gcdt_classify_regions(const int32_t* d_adj, const uint8_t
     uintptr_t d0 = (uintptr_t)d_depth, s0 = (uintptr_t)d_scratch;
     if (d0 < s0 + scratch_bytes && s0 < d0 + 4 * (size_t)n_tris) return GCDT_BAD_INPUT;
 
+    const uintptr_t d1 = d0 + 4 * (size_t)n_tris, a0 = (uintptr_t)d_adj, f0 = (uintptr_t)d_cflags;
+    const bool over_inputs = (d0 < a0 + 12 * (size_t)n_tris && a0 < d1) || (d0 < f0 + (size_t)n_tris && f0 < d1);
+    int* list = over_inputs ? level : d_depth;
+
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned grid = (unsigned)((n_tris + kBlock - 1) / kBlock);
     const unsigned tiles = (unsigned)((n_tris + kTileTris - 1) / kTileTris);
     const unsigned xgrid = (unsigned)((n_tris + kBlock * kExpandItems - 1) / (kBlock * kExpandItems));
     const unsigned lgrid = grid < 2048 ? grid : 2048;   // list passes: the length is only known on the device
     cudaError_t e = cudaMemsetAsync(flags, 0, 4 * sizeof(int), st);
-    if (e == cudaSuccess) { k_tile<<<tiles, kTileBlock, 0, st>>>(d_adj, d_cflags, n_tris, parent, d_depth, flags); e = cudaGetLastError(); }
-    if (e == cudaSuccess) { k_join<<<lgrid, kBlock, 0, st>>>(d_adj, d_cflags, n_tris, d_depth, parent, flags); e = cudaGetLastError(); }
+    if (e == cudaSuccess) { k_tile<<<tiles, kTileBlock, 0, st>>>(d_adj, d_cflags, n_tris, parent, list, flags); e = cudaGetLastError(); }
+    if (e == cudaSuccess) { k_join<<<lgrid, kBlock, 0, st>>>(d_adj, d_cflags, n_tris, list, parent, flags); e = cudaGetLastError(); }
     if (e == cudaSuccess) { k_compress<<<grid, kBlock, 0, st>>>(n_tris, parent, level, flags); e = cudaGetLastError(); }
-    if (e == cudaSuccess) { k_seed<<<lgrid, kBlock, 0, st>>>(d_adj, d_depth, flags, parent, level); e = cudaGetLastError(); }
+    if (e == cudaSuccess) {
+        if (over_inputs) k_seed_all<<<grid, kBlock, 0, st>>>(d_adj, n_tris, parent, level);
+        else k_seed<<<lgrid, kBlock, 0, st>>>(d_adj, list, flags, parent, level);
+        e = cudaGetLastError();
+    }
 
     // Breadth-first rounds, two per read-back: round L + 1 finds nothing to
     // do when round L reached nothing new, and most meshes end there (depth

@@ -200,8 +200,17 @@ def test_gpu_classification_across_tiles(rings, npts, shuffled):
         cf = np.ascontiguousarray(cf[old])
     want, wmd = regions.region_depth(adj, cf)
     assert wmd == rings
-    depth, md = g.classify_regions(torch.from_numpy(np.ascontiguousarray(adj)).cuda(), torch.from_numpy(cf).cuda())
+    d_adj, d_cf = torch.from_numpy(np.ascontiguousarray(adj)).cuda(), torch.from_numpy(cf).cuda()
+    depth, md = g.classify_regions(d_adj, d_cf)
     assert md == wmd and np.array_equal(depth.cpu().numpy(), want)
+    # the result may lie over the adjacency, which is read before it is written
+    L, T = g.lib(), len(adj)
+    scratch = torch.empty(int(L.gcdt_classify_regions_scratch_bytes(T)), dtype=torch.uint8, device="cuda")
+    p = lambda x: ctypes.c_void_p(x.data_ptr())
+    over = d_adj.view(-1)[T:2 * T]
+    assert L.gcdt_classify_regions(p(d_adj), p(d_cf), T, p(over), None, p(scratch), scratch.numel(), None) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(over.cpu().numpy(), want)
 
 
 @pytest.mark.gpu
